@@ -100,7 +100,6 @@ static void free_sim(ss_sim* s) {
     cudaFree(s->cmat_alpha);
     cudaFree(s->cmat_state);
     cudaFree(s->cmat_part);
-    cudaFree(s->cluster_fine);
     for (auto& g : s->graphs)
         if (g.exec) cudaGraphExecDestroy(g.exec);
     cudaFree(s->d_scale);
@@ -212,9 +211,9 @@ int ss_create(const ss_desc* d, void* stream, ss_sim** out) {
     // dependent launch (each waits for the previous one to finish before it
     // is scheduled); the results are the same.
     if (const char* e = getenv("SMOKESIM_PDL")) s->pdl = atoi(e) ? 1 : 0;
-    // SMOKESIM_CLUSTER=0 runs the mixed solve's small coarse levels as one
-    // launch per level operation instead of one thread-block cluster launch;
-    // the results are the same.
+    // SMOKESIM_CLUSTER=0 runs the small coarse levels in one thread block, and
+    // those that do not fit it as one launch per level operation, instead of one
+    // thread-block cluster launch; the results are the same.
     if (const char* e = getenv("SMOKESIM_CLUSTER")) s->use_cluster = atoi(e) ? 1 : 0;
     // SMOKESIM_DEVICE_LOOP=0 runs the mixed solve's tolerance loop on the
     // host, reading the residual back after every refinement step, instead of
@@ -246,9 +245,8 @@ int ss_create(const ss_desc* d, void* stream, ss_sim** out) {
         s->lv[l].hh = s->lv[l].h * s->lv[l].h;
     }
     s->bottom = bottom_start(s);
-    s->cluster_from = coarse_cluster_from(s);
 
-    int rc = SS_OK;
+    int rc = coarse_setup(s);
     auto A = [&](void** p, size_t bytes) { if (rc == SS_OK) rc = dalloc(p, bytes); };
     for (int dd = 0; dd < s->dim; ++dd)
         for (int b = 0; b < 2; ++b) A((void**)&s->vel[dd][b], s->nv[dd] * sizeof(float));
@@ -262,9 +260,9 @@ int ss_create(const ss_desc* d, void* stream, ss_sim** out) {
         const size_t n = (size_t)s->lv[l].n[0] * s->lv[l].n[1] * s->lv[l].n[2];
         A((void**)&s->p[l], n * sizeof(float));
         A((void**)&s->r[l], n * sizeof(float));
-        if (l < s->bottom || l == 0) A((void**)&s->p_alt[l], n * sizeof(float));
+        if (l < s->coarse_from || l == 0) A((void**)&s->p_alt[l], n * sizeof(float));
         if (l > 0) A((void**)&s->alpha[l], n * sizeof(float));
-        if (l > 0 && l < s->bottom) A((void**)&s->r_alt[l], n * sizeof(float));
+        if (l > 0 && l < s->coarse_from) A((void**)&s->r_alt[l], n * sizeof(float));
     }
     A((void**)&s->div0, s->ncell * sizeof(float));
     if (s->enclosed) s->div0r = s->div0;
@@ -640,8 +638,19 @@ int ss_set_level(ss_sim* s, int L, int what, const float* host, size_t count, vo
 }
 
 // ------------------------------------------------------------------ solver
-// v_cycle (common/physics/grid.c:177-209).  Levels from s->bottom down run in
-// one single-block launch; above it every red-black sweep is one tiled launch,
+static int v_cycle_rec(ss_sim* s, const StepConsts& c, const ss_mg_schedule& mg, int L, cudaStream_t st);
+
+// The V-cycle of level L from a zero pressure.  The cluster's levels start
+// from zero themselves; the others clear the array.
+static int coarse_correction(ss_sim* s, const StepConsts& c, const ss_mg_schedule& mg, int L, cudaStream_t st) {
+    if (L >= s->coarse_from) return launch_coarse(s, mg, L, st, true);
+    const size_t nc = (size_t)s->lv[L].n[0] * s->lv[L].n[1] * s->lv[L].n[2];
+    CU(cudaMemsetAsync(s->p[L], 0, nc * sizeof(float), st), "clear coarse p");
+    return v_cycle_rec(s, c, mg, L, st);
+}
+
+// v_cycle (common/physics/grid.c:177-209).  Levels from s->coarse_from down run
+// in one cluster launch; above it every red-black sweep is one tiled launch,
 // the last pre-smoothing sweep carrying the residual + restriction and the
 // first post-smoothing sweep the prolongation.
 static int v_cycle_rec(ss_sim* s, const StepConsts& c, const ss_mg_schedule& mg, int L, cudaStream_t st) {
@@ -650,20 +659,16 @@ static int v_cycle_rec(ss_sim* s, const StepConsts& c, const ss_mg_schedule& mg,
         // level 0 on the colour-split arrays; residual + restriction fused
         TRY(launch_rb_sweep(s, mg.n_pre, st));
         TRY(launch_rb_residual_restrict(s, st));
-        const size_t nc = (size_t)s->lv[1].n[0] * s->lv[1].n[1] * s->lv[1].n[2];
-        CU(cudaMemsetAsync(s->p[1], 0, nc * sizeof(float), st), "clear coarse p");
-        TRY(v_cycle_rec(s, c, mg, 1, st));
+        TRY(coarse_correction(s, c, mg, 1, st));
         TRY(launch_rb_prolong(s, st));
         return launch_rb_sweep(s, mg.n_post, st);
     }
-    if (L >= 1 && L >= s->bottom && L < s->levels) return launch_bottom(s, mg, L, st);
+    if (L >= 1 && L >= s->coarse_from && L < s->levels) return launch_coarse(s, mg, L, st);
     if (L == s->levels - 1) return launch_smooth(s, c, L, mg.n_coarse, q, st);
     for (int i = 0; i < mg.n_pre; ++i) TRY(launch_rbgs_sweep(s, c, L, q, false, i == mg.n_pre - 1, st));
     // residual written in place only where the reference's post-smoother reads it
     if (mg.n_pre == 0) TRY(launch_residual(s, c, L, q && L > 0, true, q, st));
-    const size_t nc = (size_t)s->lv[L + 1].n[0] * s->lv[L + 1].n[1] * s->lv[L + 1].n[2];
-    CU(cudaMemsetAsync(s->p[L + 1], 0, nc * sizeof(float), st), "clear coarse p");
-    TRY(v_cycle_rec(s, c, mg, L + 1, st));
+    TRY(coarse_correction(s, c, mg, L + 1, st));
     if (mg.n_post == 0) return launch_prolong(s, L, st);
     for (int i = 0; i < mg.n_post; ++i) TRY(launch_rbgs_sweep(s, c, L, q, i == 0, false, st));
     return SS_OK;
@@ -720,7 +725,7 @@ static int ensure_pyramid(ss_sim* s, cudaStream_t st) {
 // launches bake in besides the simulation's own (stable) buffers.  Runs the
 // body directly on the legacy stream or when the caller is capturing.
 struct GraphKey {
-    int kind, parity, slot, rb, bottom;
+    int kind, parity, slot, rb, coarse;
     ss_mg_schedule mg;
     float dt, rho;
 };
@@ -769,7 +774,7 @@ static int run_graph(ss_sim* s, int which, const GraphKey& key, cudaStream_t st,
 static GraphKey graph_key(const ss_sim* s, int kind, int parity, int slot, int rb, const ss_params* p) {
     GraphKey k;
     memset(&k, 0, sizeof k);
-    k.kind = kind; k.parity = parity; k.slot = slot; k.rb = rb; k.bottom = s->bottom;
+    k.kind = kind; k.parity = parity; k.slot = slot; k.rb = rb; k.coarse = s->coarse_from;
     k.mg = p->mg;
     k.dt = p->time_step; k.rho = p->density;
     return k;
@@ -808,7 +813,7 @@ static int ensure_mixed(ss_sim* s, int prec, cudaStream_t st) {
             CU(cudaMemsetAsync(s->cr[l], 0, n * 2, st), "memset");
         }
     }
-    if (s->coarse_matrix && !s->cmat && s->bottom <= s->levels - 1) {
+    if (s->coarse_matrix && !s->cmat && s->coarse_from <= s->levels - 1) {
         const ss::Level& lc = s->lv[s->levels - 1];
         const long long nc = (long long)lc.n[0] * lc.n[1] * lc.n[2];
         if (nc <= kCoarseResponseMax) {
@@ -822,7 +827,6 @@ static int ensure_mixed(ss_sim* s, int prec, cudaStream_t st) {
             s->cmat_iters = -1;
         }
     }
-    TRY(coarse_cluster_setup(s));
     s->cstore = prec;
     return SS_OK;
 }
@@ -840,8 +844,7 @@ static int v_cycle_mixed(ss_sim* s, const StepConsts& c, const ss_mg_schedule& m
         TRY(launch_rb_prolong_mixed(s, prec, st));
         return launch_rb_sweep(s, mg.n_post, st, z);
     }
-    if (L == s->cluster_from && s->cluster_ctas > 0) return coarse_cluster(s, mg, L, prec, st);
-    if (L >= s->bottom) return coarse_bottom(s, mg, L, prec, st);
+    if (L >= s->coarse_from) return launch_coarse_mixed(s, mg, L, prec, st);
     if (L == s->levels - 1) return coarse_smooth(s, c, L, mg.n_coarse, prec, st);
     TRY(coarse_smooth(s, c, L, mg.n_pre, prec, st));
     TRY(coarse_residual_restrict(s, c, L, prec, st));   // also clears level L+1's p

@@ -1272,7 +1272,7 @@ static int adj_sweeps(ss_sim* s, const AdjLevel& a, int L, int iterations, cudaS
 }
 
 // ------------------------------------------------ single-block lower V-cycle^T
-// The transpose of k_bottom: levels Lb..coarsest in one thread block with the
+// The transpose of the lower V-cycle: levels Lb..coarsest in one thread block with the
 // adjoint arrays (pbar, bbar, T of every level) in shared memory - the
 // 2*n_coarse + 1 launches of the coarsest level's transposed sweeps alone
 // would otherwise dominate.  Same per-cell operations as the level kernels
@@ -1535,6 +1535,19 @@ __global__ void __launch_bounds__(1024) k_adj_bottom(AdjBottomArgs b) {
         b.pbar0[c] = sp[c];
         b.bbar0[c] += sb[c];
     }
+}
+
+int bottom_start(const ss_sim* s) {
+    // finest level >= 1 from which the rest of the pyramid fits the block's shared memory
+    long long cum = 0;
+    int start = s->levels;
+    for (int l = s->levels - 1; l >= 1; --l) {
+        const long long n = (long long)s->lv[l].n[0] * s->lv[l].n[1] * s->lv[l].n[2];
+        if ((cum + n) * 12 > kBottomSmemBytes) break;
+        cum += n;
+        start = l;
+    }
+    return start;
 }
 
 static int adj_bottom(ss_sim* s, const ss_mg_schedule& mg, int L, const AdjScratch& w, cudaStream_t st) {

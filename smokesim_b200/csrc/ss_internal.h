@@ -109,7 +109,7 @@ struct ss_sim {
     int svel_active = 0;
 
     int levels = 0;
-    int bottom = 0;            // first level solved by the single-block bottom kernel (== levels: none)
+    int bottom = 0;            // first level of the adjoint's single-block lower V-cycle (== levels: none)
     ss::Level lv[SS_MAX_LEVELS];
     float* p[SS_MAX_LEVELS] = {};
     float* r[SS_MAX_LEVELS] = {};
@@ -185,13 +185,12 @@ struct ss_sim {
     cudaStream_t chain_stream = nullptr;   // records the nested step graphs
     // programmatic dependent launch of the solve's kernel chain (SMOKESIM_PDL=0 sets 0)
     int pdl = 1;
-    // mixed solve: the levels from cluster_from down in one thread-block
-    // cluster launch (k_coarse_cluster) of cluster_ctas CTAs; -1 = not yet
-    // probed, 0 = per-level launches (SMOKESIM_CLUSTER=0 sets use_cluster 0)
+    // the V-cycle's levels from coarse_from down run in one thread-block cluster
+    // launch (k_coarse.cu) of at most coarse_max_ctas CTAs
+    // (SMOKESIM_CLUSTER=0 sets use_cluster 0: one CTA, fewer levels)
     int use_cluster = 1;
-    int cluster_from = 0;
-    int cluster_ctas = -1;
-    float* cluster_fine = nullptr;   // a cluster level's residuals (kClusterCells floats)
+    int coarse_from = 0;
+    int coarse_max_ctas = 1;
     int rb_active = 0;         // level-0 pressure currently lives colour-split in p_alt[0]
     std::vector<ss::TensorMapEntry> tmaps;
     cudaStream_t stream0 = nullptr;
@@ -229,10 +228,14 @@ int launch_restrict(ss_sim* s, int L, cudaStream_t st);
 int launch_prolong(ss_sim* s, int L, cudaStream_t st);
 int launch_projected_residual_norm(ss_sim* s, const StepConsts& c, int slot, cudaStream_t st);
 int launch_solid_pyramid(ss_sim* s, cudaStream_t st);
-// levels Lb..coarsest of the V-cycle in one thread block (shared memory)
+// levels L..coarsest of the V-cycle in one cluster launch (k_coarse.cu), L >=
+// coarse_from; p_zero: level L's pressure is 0 whatever its array holds
+int coarse_setup(ss_sim* s);
+int launch_coarse(ss_sim* s, const ss_mg_schedule& mg, int L, cudaStream_t st, bool p_zero = false);
+int launch_coarse_mixed(ss_sim* s, const ss_mg_schedule& mg, int L, int prec, cudaStream_t st);
+// the adjoint's single-block lower V-cycle
 constexpr int kBottomSmemBytes = 160 * 1024;
 int bottom_start(const ss_sim* s);
-int launch_bottom(ss_sim* s, const ss_mg_schedule& mg, int L, cudaStream_t st);
 // one red-black sweep per launch, tiled in shared memory (k_rbgs.cu)
 int launch_rbgs_sweep(ss_sim* s, const StepConsts& c, int L, int quirks, bool prolong, bool resid,
                       cudaStream_t st);
@@ -256,10 +259,6 @@ int rb_init_vector_paths(ss_sim* s, cudaStream_t st);
 int coarse_smooth(ss_sim* s, const StepConsts& c, int L, int iterations, int prec, cudaStream_t st);
 int coarse_residual_restrict(ss_sim* s, const StepConsts& c, int L, int prec, cudaStream_t st);
 int coarse_prolong(ss_sim* s, int L, int prec, cudaStream_t st);
-int coarse_bottom(ss_sim* s, const ss_mg_schedule& mg, int L, int prec, cudaStream_t st);
-int coarse_cluster_from(const ss_sim* s);
-int coarse_cluster_setup(ss_sim* s);
-int coarse_cluster(ss_sim* s, const ss_mg_schedule& mg, int L, int prec, cudaStream_t st);
 int launch_rb_residual_restrict_mixed(ss_sim* s, int prec, cudaStream_t st);
 
 int launch_rb_prolong_mixed(ss_sim* s, int prec, cudaStream_t st);
