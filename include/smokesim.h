@@ -217,14 +217,11 @@ int ss_clear_grid(ss_sim* sim, float t_ambient, void* stream);
 /* ---- the step ------------------------------------------------------------------ */
 /* Reference run_physics_step (common/physics/physics.c:72-101), nsteps times. */
 int ss_run_physics_step(ss_sim* sim, const ss_params* params, int nsteps, void* stream);
-/* Statistics of the last ss_run_physics_step call.  Every bounded wait inside
- * a kernel that gave up (bit 0 of the simulation's device error word: a
- * coarse-level sweep whose TMA tile loads did not arrive in time) is reported
- * as SS_E_CUDA by the next call that reads the device back - ss_get_stats,
- * ss_get_field with a host destination, or the step itself when it collects
- * statistics or solves to a tolerance - and then cleared.  A step that neither
+/* Statistics of the last ss_run_physics_step call.  A step that neither
  * collects statistics nor solves to a tolerance returns SS_OK before its
- * kernels ran, so check one of those calls before trusting its fields. */
+ * kernels ran: a CUDA error of theirs is reported by the next call that waits
+ * for the device (ss_get_field with a host destination, or the step itself when
+ * it collects statistics or solves to a tolerance). */
 int ss_get_stats(ss_sim* sim, ss_stats* out);
 
 /* ---- individual stages (reference common/physics/grid.h:37-68) -------------- */

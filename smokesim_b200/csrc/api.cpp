@@ -61,9 +61,6 @@ StepConsts make_consts(const ss_sim* s, const ss_params* p) {
 #define CU(x, what) TRY(check_cuda((x), what))
 
 static cudaStream_t as_stream(void* st) { return (cudaStream_t)st; }
-extern "C" {
-static int check_device_error(ss_sim* s, cudaStream_t st);
-}
 
 static int dalloc(void** p, size_t bytes) {
     if (bytes == 0) bytes = 16;
@@ -82,8 +79,8 @@ static void free_sim(ss_sim* s) {
     for (int d = 0; d < 3; ++d) cudaFree(s->svel[d]);
     for (int l = 0; l < s->levels; ++l) {
         cudaFree(s->p[l]); cudaFree(s->r[l]); cudaFree(s->alpha[l]);
-        cudaFree(s->p_alt[l]); cudaFree(s->r_alt[l]);
     }
+    cudaFree(s->p_alt);
     cudaFree(s->div0);
     if (s->div0r != s->div0) cudaFree(s->div0r);
     cudaFree(s->vort);
@@ -202,10 +199,6 @@ int ss_create(const ss_desc* d, void* stream, ss_sim** out) {
     s->h = d->cell_size;
     s->t_amb0 = d->t_ambient;
     s->ncell = (size_t)s->nx * s->ny * s->nz;
-    // SMOKESIM_TMA=0 keeps the coarse-level tiled sweeps on per-thread loads
-    // (the form every grid whose rows TMA cannot tile takes anyway); the
-    // default 1 feeds them with TMA.  The results are the same.
-    if (const char* e = getenv("SMOKESIM_TMA")) s->use_tma = atoi(e) ? 1 : 0;
     if (const char* e = getenv("SMOKESIM_COARSE_SWEEPS")) s->coarse_matrix = atoi(e) ? 0 : 1;
     // SMOKESIM_PDL=0 launches the solve's kernels without programmatic
     // dependent launch (each waits for the previous one to finish before it
@@ -260,9 +253,7 @@ int ss_create(const ss_desc* d, void* stream, ss_sim** out) {
         const size_t n = (size_t)s->lv[l].n[0] * s->lv[l].n[1] * s->lv[l].n[2];
         A((void**)&s->p[l], n * sizeof(float));
         A((void**)&s->r[l], n * sizeof(float));
-        if (l < s->coarse_from || l == 0) A((void**)&s->p_alt[l], n * sizeof(float));
         if (l > 0) A((void**)&s->alpha[l], n * sizeof(float));
-        if (l > 0 && l < s->coarse_from) A((void**)&s->r_alt[l], n * sizeof(float));
     }
     A((void**)&s->div0, s->ncell * sizeof(float));
     if (s->enclosed) s->div0r = s->div0;
@@ -271,6 +262,7 @@ int ss_create(const ss_desc* d, void* stream, ss_sim** out) {
     if (s->dim == 2) A((void**)&s->vort, s->ncell * sizeof(float));
     A((void**)&s->fmask, s->ncell);   // level-0 fluid mask (k_rb.cu, k_mixed.cu, k_adjoint.cu)
     if (s->nx % 2 == 0 && s->levels > 1) {   // colour-split level 0 (k_rb.cu)
+        A((void**)&s->p_alt, s->ncell * sizeof(float));
         A((void**)&s->rhs_s, s->ncell * sizeof(float));
         A((void**)&s->rhs_r, s->ncell * sizeof(float));
         A((void**)&s->rb_mask, s->ncell);
@@ -280,7 +272,6 @@ int ss_create(const ss_desc* d, void* stream, ss_sim** out) {
     s->red.stage2 = s->red.max_blocks / 1024 + 2;
     A((void**)&s->red.partial2, (size_t)2 * s->red.stage2 * sizeof(double));
     A((void**)&s->red.out, SLOT_COUNT * sizeof(double));
-    if (rc == SS_OK) s->d_err = reinterpret_cast<int*>(s->red.out + SLOT_ERR);
     A((void**)&s->red.ticket, sizeof(unsigned int));
     if (rc == SS_OK) {
         cudaError_t e = cudaMallocHost((void**)&s->red.host, SLOT_COUNT * sizeof(double));
@@ -558,7 +549,7 @@ int ss_get_field(ss_sim* s, int f, float* host, size_t count, void* stream) {
     if (count != n) return set_error(SS_E_INVALID, "element count does not match the field");
     CU(cudaMemcpyAsync(host, d, n * sizeof(float), cudaMemcpyDeviceToHost, st), "get_field");
     CU(cudaStreamSynchronize(st), "get_field sync");
-    return check_device_error(s, st);
+    return SS_OK;
 }
 
 int ss_field_device_ptr(ss_sim* s, int f, void** dptr, size_t* count) {
@@ -638,76 +629,40 @@ int ss_set_level(ss_sim* s, int L, int what, const float* host, size_t count, vo
 }
 
 // ------------------------------------------------------------------ solver
-static int v_cycle_rec(ss_sim* s, const StepConsts& c, const ss_mg_schedule& mg, int L, cudaStream_t st);
-
-// The V-cycle of level L from a zero pressure.  The cluster's levels start
-// from zero themselves; the others clear the array.
-static int coarse_correction(ss_sim* s, const StepConsts& c, const ss_mg_schedule& mg, int L, cudaStream_t st) {
-    if (L >= s->coarse_from) return launch_coarse(s, mg, L, st, true);
-    const size_t nc = (size_t)s->lv[L].n[0] * s->lv[L].n[1] * s->lv[L].n[2];
-    CU(cudaMemsetAsync(s->p[L], 0, nc * sizeof(float), st), "clear coarse p");
-    return v_cycle_rec(s, c, mg, L, st);
-}
-
 // v_cycle (common/physics/grid.c:177-209).  Levels from s->coarse_from down run
-// in one cluster launch; above it every red-black sweep is one tiled launch,
-// the last pre-smoothing sweep carrying the residual + restriction and the
-// first post-smoothing sweep the prolongation.
-static int v_cycle_rec(ss_sim* s, const StepConsts& c, const ss_mg_schedule& mg, int L, cudaStream_t st) {
+// in one cluster launch; above it every half-sweep, residual + restriction and
+// prolongation is one launch.  Two colours a launch on shared-memory tiles, with
+// the neighbouring operations fused in, took longer at every size: a tile's
+// halo is updated again and its blocks are few (64^3 level, per V-cycle: 58
+// against 35 us; 97x75x61 level 0: 85 against 49).
+// p_zero: level L starts from a zero pressure (cleared by the restriction where
+// its launches read the array).
+static int v_cycle_rec(ss_sim* s, const StepConsts& c, const ss_mg_schedule& mg, int L, cudaStream_t st,
+                       bool p_zero = false) {
     const int q = mg.ref_quirks;
     if (L == 0 && s->rb_active) {
         // level 0 on the colour-split arrays; residual + restriction fused
         TRY(launch_rb_sweep(s, mg.n_pre, st));
         TRY(launch_rb_residual_restrict(s, st));
-        TRY(coarse_correction(s, c, mg, 1, st));
+        TRY(v_cycle_rec(s, c, mg, 1, st, true));
         TRY(launch_rb_prolong(s, st));
         return launch_rb_sweep(s, mg.n_post, st);
     }
-    if (L >= 1 && L >= s->coarse_from && L < s->levels) return launch_coarse(s, mg, L, st);
+    if (L >= s->coarse_from) return launch_coarse(s, mg, L, st, p_zero);
     if (L == s->levels - 1) return launch_smooth(s, c, L, mg.n_coarse, q, st);
-    for (int i = 0; i < mg.n_pre; ++i) TRY(launch_rbgs_sweep(s, c, L, q, false, i == mg.n_pre - 1, st));
+    TRY(launch_smooth(s, c, L, mg.n_pre, q, st));
     // residual written in place only where the reference's post-smoother reads it
-    if (mg.n_pre == 0) TRY(launch_residual(s, c, L, q && L > 0, true, q, st));
-    TRY(coarse_correction(s, c, mg, L + 1, st));
-    if (mg.n_post == 0) return launch_prolong(s, L, st);
-    for (int i = 0; i < mg.n_post; ++i) TRY(launch_rbgs_sweep(s, c, L, q, i == 0, false, st));
-    return SS_OK;
+    TRY(launch_residual(s, c, L, q && L > 0, true, q, st));
+    TRY(v_cycle_rec(s, c, mg, L + 1, st, true));
+    TRY(launch_prolong(s, L, st));
+    return launch_smooth(s, c, L, mg.n_post, q, st);
 }
 
-// The device error word collects the bounded waits that gave up (bit 0: a
-// coarse-level sweep's TMA tile load did not arrive in time, so that sweep
-// skipped its cells).  Only those sweeps (the FP32 solve's coarse levels) set
-// it; a solve that may run them arms s->err_armed.  It is read - with the
-// statistics slots of a step, which hold it, and by ss_get_stats and
-// ss_get_field while armed - reported once and cleared, so the next report
-// concerns later launches only.
-static int report_device_error(ss_sim* s, int err, cudaStream_t st) {
-    s->err_armed = 0;
-    if (err) {
-        CU(cudaMemsetAsync(s->d_err, 0, sizeof(int), st), "error word clear");
-        CU(cudaStreamSynchronize(st), "error word clear");
-        if (err & 1)
-            return set_error(SS_E_CUDA, "a coarse-level sweep gave up waiting for its TMA tile loads (bounded wait); "
-                                        "the pressure of that solve is not valid");
-        return set_error(SS_E_CUDA, "unknown bit set in the device error word");
-    }
-    return SS_OK;
-}
-
-static int check_device_error(ss_sim* s, cudaStream_t st) {
-    int err = 0;
-    CU(cudaMemcpyAsync(&err, s->d_err, sizeof(int), cudaMemcpyDeviceToHost, st), "error word");
-    CU(cudaStreamSynchronize(st), "error word sync");
-    return report_device_error(s, err, st);
-}
-
-// the statistics slots and the error word, in one copy and one synchronisation
+// the statistics slots, in one copy and one synchronisation
 static int read_slots(ss_sim* s, cudaStream_t st) {
     CU(cudaMemcpyAsync(s->red.host, s->red.out, SLOT_COUNT * sizeof(double), cudaMemcpyDeviceToHost, st), "slots");
     CU(cudaStreamSynchronize(st), "slots sync");
-    int err = 0;
-    memcpy(&err, &s->red.host[SLOT_ERR], sizeof(int));
-    return report_device_error(s, err, st);
+    return SS_OK;
 }
 
 static int ensure_pyramid(ss_sim* s, cudaStream_t st) {
@@ -831,7 +786,7 @@ static int ensure_mixed(ss_sim* s, int prec, cudaStream_t st) {
     return SS_OK;
 }
 
-// One V-cycle on the correction e (colour-split FP32 level 0 in p_alt[0],
+// One V-cycle on the correction e (colour-split FP32 level 0 in p_alt,
 // coarse levels FP16/BF16), corrected operators (ref_quirks = 0).
 static int v_cycle_mixed(ss_sim* s, const StepConsts& c, const ss_mg_schedule& mg, int L, int prec, cudaStream_t st) {
     if (L == 0) {
@@ -1092,7 +1047,6 @@ static int pressure_solve(ss_sim* s, const ss_params* p, const StepConsts& c, cu
     const ss_mg_schedule& mg = p->mg;
     if (mg.precision != SS_PREC_FP32) return pressure_solve_mixed(s, p, c, st, defer_p0);
     s->p64_valid = 0;
-    s->err_armed = 1;   // its coarse-level sweeps may take the bounded-wait TMA form
     const bool tol_mode = mg.tol > 0.0;
     const bool stats = p->collect_stats || tol_mode;
     TRY(ensure_pyramid(s, st));
@@ -1290,7 +1244,7 @@ int ss_set_force_field(ss_sim* s, int n, const float* field, void* stream) {
 int ss_get_stats(ss_sim* s, ss_stats* out) {
     if (!s || !out) return set_error(SS_E_INVALID, "NULL argument");
     *out = s->st;
-    return s->err_armed ? check_device_error(s, nullptr) : SS_OK;
+    return SS_OK;
 }
 
 // ------------------------------------------------------------ single stages

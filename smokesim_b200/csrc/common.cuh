@@ -333,7 +333,7 @@ SS_D float div_by_count(float a, int f) {
 
 // Fluid mask byte of a level-0 cell: bit 0 the cell is fluid, bits 1-6 the
 // +y,-y,+x,-x,+z,-z neighbour is fluid (out of grid: fluid on an open grid,
-// solid on an enclosed one).  Zero - the TMA fill outside the grid - reads as
+// solid on an enclosed one).  Zero - a load outside the grid - reads as
 // "not fluid", so tile kernels need no bounds checks.
 enum : uint8_t {
     M_FLUID = 1u << 0,

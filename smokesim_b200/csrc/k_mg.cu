@@ -127,11 +127,11 @@ __global__ void __launch_bounds__(256) k_residual_restrict(MGArgsT<T> a, T* __re
 }
 
 template <int DIM, bool L0>
-static void launch_rr(bool pdl, const MGArgs& a, float* rc, int cx, int cy, int cz, bool wf, bool wc, dim3 g, dim3 b,
-                      cudaStream_t st) {
-    if (wf && wc) launch_k(pdl, g, b, 0, st, k_residual_restrict<DIM, L0, true, true>, a, rc, cx, cy, cz, nullptr);
-    else if (wf) launch_k(pdl, g, b, 0, st, k_residual_restrict<DIM, L0, true, false>, a, rc, cx, cy, cz, nullptr);
-    else launch_k(pdl, g, b, 0, st, k_residual_restrict<DIM, L0, false, true>, a, rc, cx, cy, cz, nullptr);
+static void launch_rr(bool pdl, const MGArgs& a, float* rc, float* pz, int cx, int cy, int cz, bool wf, bool wc, dim3 g,
+                      dim3 b, cudaStream_t st) {
+    if (wf && wc) launch_k(pdl, g, b, 0, st, k_residual_restrict<DIM, L0, true, true>, a, rc, cx, cy, cz, pz);
+    else if (wf) launch_k(pdl, g, b, 0, st, k_residual_restrict<DIM, L0, true, false>, a, rc, cx, cy, cz, pz);
+    else launch_k(pdl, g, b, 0, st, k_residual_restrict<DIM, L0, false, true>, a, rc, cx, cy, cz, pz);
 }
 
 int launch_residual(ss_sim* s, const StepConsts& c, int L, bool write_fine, bool write_coarse, int quirks,
@@ -143,14 +143,16 @@ int launch_residual(ss_sim* s, const StepConsts& c, int L, bool write_fine, bool
     const int cy = write_coarse ? s->lv[L + 1].n[1] : 0;
     const int cz = write_coarse ? s->lv[L + 1].n[2] : 0;
     float* rc = write_coarse ? s->r[L + 1] : nullptr;
+    // the next level's initial guess, where its launches read it
+    float* pz = write_coarse && L + 1 < s->coarse_from ? s->p[L + 1] : nullptr;
     dim3 b(32, 8, 1);
     dim3 g = grid_for((a.nx + 1) / 2, (a.ny + 1) / 2, s->dim == 3 ? (a.nz + 1) / 2 : 1, b);
     if (s->dim == 3) {
-        if (L == 0) launch_rr<3, true>(s->pdl != 0, a, rc, cx, cy, cz, write_fine, write_coarse, g, b, st);
-        else launch_rr<3, false>(s->pdl != 0, a, rc, cx, cy, cz, write_fine, write_coarse, g, b, st);
+        if (L == 0) launch_rr<3, true>(s->pdl != 0, a, rc, pz, cx, cy, cz, write_fine, write_coarse, g, b, st);
+        else launch_rr<3, false>(s->pdl != 0, a, rc, pz, cx, cy, cz, write_fine, write_coarse, g, b, st);
     } else {
-        if (L == 0) launch_rr<2, true>(s->pdl != 0, a, rc, cx, cy, cz, write_fine, write_coarse, g, b, st);
-        else launch_rr<2, false>(s->pdl != 0, a, rc, cx, cy, cz, write_fine, write_coarse, g, b, st);
+        if (L == 0) launch_rr<2, true>(s->pdl != 0, a, rc, pz, cx, cy, cz, write_fine, write_coarse, g, b, st);
+        else launch_rr<2, false>(s->pdl != 0, a, rc, pz, cx, cy, cz, write_fine, write_coarse, g, b, st);
     }
     s->nlaunch += 1;
     return check_cuda(cudaGetLastError(), "k_residual_restrict");

@@ -292,7 +292,7 @@ int launch_ir_residual(ss_sim* s, const StepConsts& c, int slot, bool accumulate
     // to the bit: only rhs_s is written, and the level-0 residual reads it
     s->rhs_r_is_s = s->lv[0].hh == 1.0f ? 1 : 0;
     float* rhs_r = s->rhs_r_is_s ? nullptr : s->rhs_r;
-#define IR_ARGS(ACC) s->p64, s->p_alt[0], s->p64b, s->div0, s->fmask, s->nx, s->ny, s->nz, k, inv_k, inv_khh, \
+#define IR_ARGS(ACC) s->p64, s->p_alt, s->p64b, s->div0, s->fmask, s->nx, s->ny, s->nz, k, inv_k, inv_khh, \
                      s->rhs_s, rhs_r, s->red.partial, s->red.partial_max, s->red.ticket, s->red.out, slot, \
                      s->d_scale, planes, d
     if (s->dim == 3) {
@@ -325,8 +325,8 @@ int launch_ir_residual(ss_sim* s, const StepConsts& c, int slot, bool accumulate
 int launch_ir_accumulate(ss_sim* s, cudaStream_t st) {
     dim3 b(32, 8, 1);
     dim3 g = grid3(s->nx, s->ny, s->nz, b);
-    if (s->dim == 3) k_ir_accumulate<3><<<g, b, 0, st>>>(s->p64, s->p_alt[0], s->fmask, s->nx, s->ny, s->nz);
-    else k_ir_accumulate<2><<<g, b, 0, st>>>(s->p64, s->p_alt[0], s->fmask, s->nx, s->ny, s->nz);
+    if (s->dim == 3) k_ir_accumulate<3><<<g, b, 0, st>>>(s->p64, s->p_alt, s->fmask, s->nx, s->ny, s->nz);
+    else k_ir_accumulate<2><<<g, b, 0, st>>>(s->p64, s->p_alt, s->fmask, s->nx, s->ny, s->nz);
     s->nlaunch += 1;
     return check_cuda(cudaGetLastError(), "k_ir_accumulate");
 }

@@ -530,8 +530,8 @@ bool rb_supported(const ss_sim* s, int quirks) {
 int launch_rb_convert(ss_sim* s, bool split, cudaStream_t st) {
     const RBLevel g = rb_level(s);
     dim3 b(128), gr((g.nx + 127) / 128, g.ny, g.nz);
-    float* red = s->p_alt[0];
-    float* black = s->p_alt[0] + s->ncell / 2;
+    float* red = s->p_alt;
+    float* black = s->p_alt + s->ncell / 2;
     if (split) k_rb_convert<true><<<gr, b, 0, st>>>(s->p[0], red, black, g);
     else k_rb_convert<false><<<gr, b, 0, st>>>(s->p[0], red, black, g);
     s->nlaunch += 1;
@@ -549,7 +549,7 @@ int launch_rb_split_mask(ss_sim* s, cudaStream_t st) {
 int launch_rb_sweep(ss_sim* s, int iterations, cudaStream_t st, bool zero, bool from_zero) {
     const RBLevel g = rb_level(s);
     const size_t h = s->ncell / 2;
-    float* p[2] = {s->p_alt[0], s->p_alt[0] + h};
+    float* p[2] = {s->p_alt, s->p_alt + h};
     const float* rhs[2] = {s->rhs_s, s->rhs_s + h};
     const uint8_t* mask[2] = {s->rb_mask, s->rb_mask + h};
     dim3 b, gr;
@@ -566,7 +566,7 @@ int launch_rb_sweep(ss_sim* s, int iterations, cudaStream_t st, bool zero, bool 
     // clears the black array itself; otherwise both arrays are cleared first
     const bool init = from_zero && s->rb_vec && iterations > 0;
     if (from_zero && !init) {
-        const cudaError_t e = cudaMemsetAsync(s->p_alt[0], 0, s->ncell * sizeof(float), st);
+        const cudaError_t e = cudaMemsetAsync(s->p_alt, 0, s->ncell * sizeof(float), st);
         if (e != cudaSuccess) return check_cuda(e, "clear level-0 pressure");
     }
     for (int it = 0; it < iterations; ++it)
@@ -612,7 +612,7 @@ static int rb_residual_restrict_t(ss_sim* s, T* rc, const float* scale, cudaStre
     const bool p2 = pow2f(hh);
     const float ih = p2 ? 1.f / hh : 0.f;
     dim3 b, gr;
-    const float* pr = s->p_alt[0];
+    const float* pr = s->p_alt;
     const float* pb = pr + h;
     const float* rr = s->rhs_r_is_s ? s->rhs_s : s->rhs_r;
     const uint8_t* mr = s->rb_mask;
@@ -657,25 +657,27 @@ static int rb_prolong_t(ss_sim* s, const T* pc, const float* scale, cudaStream_t
         dim3 b, gr;
         row_launch(cx / 4, cy, cz, b, gr);
         if (s->dim == 3 && zero)
-            launch_k(s->pdl, gr, b, 0, st, k_rb_prolong4<3, T, true>, s->p_alt[0], s->p_alt[0] + h, g, pc, cx, cy, cz, s->rb_pw,
+            launch_k(s->pdl, gr, b, 0, st, k_rb_prolong4<3, T, true>, s->p_alt, s->p_alt + h, g, pc, cx, cy, cz, s->rb_pw,
                      scale, s->rb_mask, s->rb_mask + h);
         else if (s->dim == 3)
-            launch_k(s->pdl, gr, b, 0, st, k_rb_prolong4<3, T>, s->p_alt[0], s->p_alt[0] + h, g, pc, cx, cy, cz, s->rb_pw,
+            launch_k(s->pdl, gr, b, 0, st, k_rb_prolong4<3, T>, s->p_alt, s->p_alt + h, g, pc, cx, cy, cz, s->rb_pw,
                      scale, nullptr, nullptr);
         else
-            launch_k(s->pdl, gr, b, 0, st, k_rb_prolong4<2, T>, s->p_alt[0], s->p_alt[0] + h, g, pc, cx, cy, cz, s->rb_pw,
+            launch_k(s->pdl, gr, b, 0, st, k_rb_prolong4<2, T>, s->p_alt, s->p_alt + h, g, pc, cx, cy, cz, s->rb_pw,
                      scale, nullptr, nullptr);
         s->nlaunch += 1;
         return check_cuda(cudaGetLastError(), "k_rb_prolong4");
     }
     dim3 b(128), gr((g.nx + 127) / 128, g.ny, g.nz);
-    if (s->dim == 3) launch_k(s->pdl, gr, b, 0, st, k_rb_prolong<3, T>, s->p_alt[0], s->p_alt[0] + h, g, pc, cx, cy, cz, scale);
-    else launch_k(s->pdl, gr, b, 0, st, k_rb_prolong<2, T>, s->p_alt[0], s->p_alt[0] + h, g, pc, cx, cy, cz, scale);
+    if (s->dim == 3) launch_k(s->pdl, gr, b, 0, st, k_rb_prolong<3, T>, s->p_alt, s->p_alt + h, g, pc, cx, cy, cz, scale);
+    else launch_k(s->pdl, gr, b, 0, st, k_rb_prolong<2, T>, s->p_alt, s->p_alt + h, g, pc, cx, cy, cz, scale);
     s->nlaunch += 1;
     return check_cuda(cudaGetLastError(), "k_rb_prolong");
 }
 
-int launch_rb_residual_restrict(ss_sim* s, cudaStream_t st) { return rb_residual_restrict_t<float>(s, s->r[1], nullptr, st); }
+int launch_rb_residual_restrict(ss_sim* s, cudaStream_t st) {
+    return rb_residual_restrict_t<float>(s, s->r[1], nullptr, st, false, s->coarse_from > 1 ? s->p[1] : nullptr);
+}
 
 int launch_rb_prolong(ss_sim* s, cudaStream_t st) { return rb_prolong_t<float>(s, s->p[1], nullptr, st); }
 

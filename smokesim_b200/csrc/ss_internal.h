@@ -62,11 +62,8 @@ struct ReduceSlots {
     double* host;         // pinned mirror of out
     int max_blocks;
 };
-// SLOT_STEPS: refinement steps a device-side tolerance loop took (a double);
-// SLOT_ERR: the device error word (an int at the start of the slot), so that
-// one copy of the slots brings both back
-enum { SLOT_DIV_BEFORE = 0, SLOT_RESIDUAL = 1, SLOT_DIV_AFTER = 2, SLOT_AMAX = 3, SLOT_STEPS = 4, SLOT_ERR = 7,
-       SLOT_COUNT = 8 };
+// SLOT_STEPS: refinement steps a device-side tolerance loop took (a double)
+enum { SLOT_DIV_BEFORE = 0, SLOT_RESIDUAL = 1, SLOT_DIV_AFTER = 2, SLOT_AMAX = 3, SLOT_STEPS = 4, SLOT_COUNT = 5 };
 
 // Convergence test of the mixed solve's tolerance loop, folded into the last
 // block of the refinement residual (k_ir_residual): it records k, the
@@ -79,14 +76,6 @@ struct IrDecide {
     int k = 0;
     int more = 0;
     int active = 0;
-};
-
-struct TensorMapEntry {
-    CUtensorMap map;
-    const void* ptr;
-    bool bytes;
-    int dims[3];
-    int box[3];
 };
 
 }  // namespace ss
@@ -113,8 +102,7 @@ struct ss_sim {
     ss::Level lv[SS_MAX_LEVELS];
     float* p[SS_MAX_LEVELS] = {};
     float* r[SS_MAX_LEVELS] = {};
-    float* p_alt[SS_MAX_LEVELS] = {};   // second buffer of the tiled sweep (p_in -> p_out)
-    float* r_alt[SS_MAX_LEVELS] = {};   // second buffer of the fused in-place residual (L >= 1)
+    float* p_alt = nullptr;             // level-0 pressure colour-split (k_rb.cu)
     float* alpha[SS_MAX_LEVELS] = {};   // coarse solid fraction (L >= 1), FP16-rounded values
     float* div0 = nullptr;              // level-0 divergence, smoother boundary rule
     float* div0r = nullptr;             // residual boundary rule (== div0 when enclosed)
@@ -155,9 +143,6 @@ struct ss_sim {
 
     ss_stats st{};
     long long nlaunch = 0;     // kernels launched since the counter was reset
-    int* d_err = nullptr;      // device error word (in red.out[SLOT_ERR]): bit 0 = a bounded barrier wait gave up
-    int err_armed = 0;         // a kernel that can set the error word ran since the word was last read
-    int use_tma = 1;           // TMA tile loads of the coarse-level tiled sweeps (0: per-thread loads)
     // mixed solve: the coarsest level by its response matrix instead of its
     // n_coarse sweeps (levels of at most kCoarseResponseMax cells)
     int coarse_matrix = 1;       // SMOKESIM_COARSE_SWEEPS=1 sets 0
@@ -191,8 +176,7 @@ struct ss_sim {
     int use_cluster = 1;
     int coarse_from = 0;
     int coarse_max_ctas = 1;
-    int rb_active = 0;         // level-0 pressure currently lives colour-split in p_alt[0]
-    std::vector<ss::TensorMapEntry> tmaps;
+    int rb_active = 0;         // level-0 pressure currently lives colour-split in p_alt
     cudaStream_t stream0 = nullptr;
 };
 
@@ -236,12 +220,6 @@ int launch_coarse_mixed(ss_sim* s, const ss_mg_schedule& mg, int L, int prec, cu
 // the adjoint's single-block lower V-cycle
 constexpr int kBottomSmemBytes = 160 * 1024;
 int bottom_start(const ss_sim* s);
-// one red-black sweep per launch, tiled in shared memory (k_rbgs.cu)
-int launch_rbgs_sweep(ss_sim* s, const StepConsts& c, int L, int quirks, bool prolong, bool resid,
-                      cudaStream_t st);
-// the same sweep with the tile fetched by TMA (k_rbgs_tma.cu); 3D, nx % 16 == 0
-bool tma_sweep_supported(const ss_sim* s, int L);
-int launch_rbgs_sweep_tma(ss_sim* s, const StepConsts& c, int L, int quirks, bool resid, cudaStream_t st);
 // level 0 on colour-split arrays during a solve (k_rb.cu)
 bool rb_supported(const ss_sim* s, int quirks);
 int launch_rb_convert(ss_sim* s, bool split, cudaStream_t st);
