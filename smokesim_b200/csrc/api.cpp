@@ -111,7 +111,7 @@ static void free_sim(ss_sim* s) {
     cudaFree(s->d_em);
     cudaFree(s->d_ob);
     cudaFree(s->d_bx);
-    if (s->chain_stream) cudaStreamDestroy(s->chain_stream);
+    if (s->record_stream) cudaStreamDestroy(s->record_stream);
     delete s;
 }
 
@@ -674,55 +674,84 @@ static int ensure_pyramid(ss_sim* s, cudaStream_t st) {
 
 // ------------------------------------------------------- solve graphs
 // The multigrid part of a solve is the same sequence of launches every step
-// (same pointers, schedule and constants): it is recorded once as a CUDA
-// graph and replayed, which removes the per-launch CPU and GPU gaps of its
-// many small coarse-level kernels.  The key holds everything the recorded
-// launches bake in besides the simulation's own (stable) buffers.  Runs the
-// body directly on the legacy stream or when the caller is capturing.
+// (same pointers, schedule and constants): it is recorded as a CUDA graph and
+// replayed, which removes the per-launch CPU and GPU gaps of its many small
+// kernels.  The key holds everything the recorded launches bake in besides the
+// simulation's own (stable) buffers.  Recording and instantiating cost more than
+// the launches themselves, so a sequence is recorded when its key comes up in a
+// second solve (first frame of a new 64^3 simulation 981 -> 416 us).  It is recorded on the simulation's own stream and launched on
+// the caller's: the legacy default stream cannot be recorded, but a graph can
+// be launched on it (601x347 frame of 141 launches: 420 -> 399 us).  Runs the body
+// directly where the caller is recording the stream.
 struct GraphKey {
     int kind, parity, slot, rb, coarse;
     ss_mg_schedule mg;
     float dt, rho;
 };
 
+// whether st takes graph launches now
+static bool graphs_ok(ss_sim* s, cudaStream_t st) {
+    if (!s->use_graphs) return false;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &cs) != cudaSuccess) {
+        cudaGetLastError();   // the legacy stream while another stream is recorded
+        return false;
+    }
+    return cs == cudaStreamCaptureStatusNone;
+}
+
+static int record_stream(ss_sim* s, cudaStream_t* out) {
+    if (!s->record_stream)
+        CU(cudaStreamCreateWithFlags(&s->record_stream, cudaStreamNonBlocking), "cudaStreamCreate(record)");
+    *out = s->record_stream;
+    return SS_OK;
+}
+
+// the slot's graph for this key: 1 ready, 0 to be recorded (an old one is
+// dropped), -1 no solve before this one has seen the key
+static int graph_state(const ss_sim* s, ss_sim::SolveGraph& g, const GraphKey& key) {
+    static_assert(sizeof(GraphKey) <= sizeof(g.key), "graph key size");
+    unsigned char kb[sizeof(g.key)] = {};
+    memcpy(kb, &key, sizeof(GraphKey));
+    if (g.seen && memcmp(g.key, kb, sizeof kb) == 0) return g.exec ? 1 : g.seen < s->solves ? 0 : -1;
+    if (g.exec) cudaGraphExecDestroy(g.exec);
+    g.exec = nullptr;
+    memcpy(g.key, kb, sizeof kb);
+    g.seen = s->solves;
+    return -1;
+}
+
+// body(stream) launches the sequence
 template <typename F>
 static int run_graph(ss_sim* s, int which, const GraphKey& key, cudaStream_t st, F body) {
-    if (!s->use_graphs || st == nullptr) return body();
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    CU(cudaStreamIsCapturing(st, &cs), "cudaStreamIsCapturing");
-    if (cs != cudaStreamCaptureStatusNone) return body();
-    static_assert(sizeof(GraphKey) <= sizeof(s->graphs[0].key), "graph key size");
-    unsigned char kb[sizeof(s->graphs[0].key)] = {};
-    memcpy(kb, &key, sizeof(GraphKey));
+    if (!graphs_ok(s, st)) return body(st);
     ss_sim::SolveGraph& g = s->graphs[which];
-    if (g.exec && memcmp(g.key, kb, sizeof kb) == 0) {
-        CU(cudaGraphLaunch(g.exec, st), "cudaGraphLaunch");
-        s->nlaunch += g.launches;
-        return SS_OK;
+    const int state = graph_state(s, g, key);
+    if (state < 0) return body(st);
+    if (state == 0) {
+        const long long before = s->nlaunch;
+        cudaStream_t cs;
+        TRY(record_stream(s, &cs));
+        CU(cudaStreamBeginCapture(cs, cudaStreamCaptureModeRelaxed), "cudaStreamBeginCapture");
+        const int rc = body(cs);
+        cudaGraph_t graph = nullptr;
+        const cudaError_t e = cudaStreamEndCapture(cs, &graph);
+        g.launches = s->nlaunch - before;
+        s->nlaunch = before;
+        if (rc != SS_OK) {
+            if (graph) cudaGraphDestroy(graph);
+            return rc;
+        }
+        CU(e, "cudaStreamEndCapture");
+        const cudaError_t ei = cudaGraphInstantiate(&g.exec, graph, 0);
+        cudaGraphDestroy(graph);
+        if (ei != cudaSuccess) {
+            g.exec = nullptr;
+            return check_cuda(ei, "cudaGraphInstantiate");
+        }
     }
-    if (g.exec) {
-        cudaGraphExecDestroy(g.exec);
-        g.exec = nullptr;
-    }
-    const long long before = s->nlaunch;
-    CU(cudaStreamBeginCapture(st, cudaStreamCaptureModeRelaxed), "cudaStreamBeginCapture");
-    const int rc = body();
-    cudaGraph_t graph = nullptr;
-    const cudaError_t e = cudaStreamEndCapture(st, &graph);
-    if (rc != SS_OK) {
-        if (graph) cudaGraphDestroy(graph);
-        return rc;
-    }
-    CU(e, "cudaStreamEndCapture");
-    const cudaError_t ei = cudaGraphInstantiate(&g.exec, graph, 0);
-    cudaGraphDestroy(graph);
-    if (ei != cudaSuccess) {
-        g.exec = nullptr;
-        return check_cuda(ei, "cudaGraphInstantiate");
-    }
-    memcpy(g.key, kb, sizeof kb);
-    g.launches = s->nlaunch - before;
     CU(cudaGraphLaunch(g.exec, st), "cudaGraphLaunch");
+    s->nlaunch += g.launches;
     return SS_OK;
 }
 
@@ -845,9 +874,8 @@ constexpr int kChainDepth = 8;
 
 static int build_solve_chain(ss_sim* s, const StepConsts& c, const ss_mg_schedule& mg, int depth,
                              ss_sim::SolveGraph& g) {
-    if (!s->chain_stream)
-        CU(cudaStreamCreateWithFlags(&s->chain_stream, cudaStreamNonBlocking), "cudaStreamCreate(chain)");
-    cudaStream_t cs = s->chain_stream;
+    cudaStream_t cs;
+    TRY(record_stream(s, &cs));
     double* const pa = s->p64;
     double* const pb = s->p64b;
     const int pdl = s->pdl;
@@ -912,34 +940,18 @@ static int build_solve_chain(ss_sim* s, const StepConsts& c, const ss_mg_schedul
     return SS_OK;
 }
 
-// The device-side loop needs a stream that graphs can be launched on and that
-// is not being recorded by the caller.
-static bool chain_ok(ss_sim* s, cudaStream_t st) {
-    if (!s->device_loop || !s->use_graphs || st == nullptr) return false;
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(st, &cs) != cudaSuccess) return false;
-    return cs == cudaStreamCaptureStatusNone;
-}
-
 // Runs up to depth refinement steps of the tolerance loop on the device and
 // reads the statistics slots once; *k = the steps it took.  The FP64 buffers
 // end swapped after an odd number of steps.
-static int run_solve_chain(ss_sim* s, const ss_params* p, const StepConsts& c, int depth, cudaStream_t st,
+// state: graph_state of its graph (chain_state below), not -1.
+static int run_solve_chain(ss_sim* s, const ss_params* p, const StepConsts& c, int depth, int state, cudaStream_t st,
                            int* k_out) {
-    const GraphKey key = graph_key(s, 4, s->p64_parity, SLOT_RESIDUAL, depth, p);
-    unsigned char kb[sizeof(s->graphs[0].key)] = {};
-    memcpy(kb, &key, sizeof(GraphKey));
     ss_sim::SolveGraph& g = s->graphs[4 + s->p64_parity];
-    if (!g.exec || memcmp(g.key, kb, sizeof kb) != 0) {
-        if (g.exec) {
-            cudaGraphExecDestroy(g.exec);
-            g.exec = nullptr;
-        }
+    if (state == 0) {
         const long long n0 = s->nlaunch;
         const int rc = build_solve_chain(s, c, p->mg, depth, g);
         s->nlaunch = n0;
         if (rc != SS_OK) return rc;
-        memcpy(g.key, kb, sizeof kb);
     }
     CU(cudaGraphLaunch(g.exec, st), "cudaGraphLaunch(solve chain)");
     TRY(read_slots(s, st));
@@ -954,6 +966,15 @@ static int run_solve_chain(ss_sim* s, const ss_params* p, const StepConsts& c, i
     }
     *k_out = k;
     return SS_OK;
+}
+
+static int chain_state(ss_sim* s, const ss_params* p, int depth, cudaStream_t st) {
+    if (!s->device_loop || !graphs_ok(s, st)) return -1;
+    // the chain is recorded by the first solve: a host loop of 46 launches and a
+    // read-back a step costs it more (two frames of a new 128^3 rollout 8.8
+    // against 10.3 ms)
+    const int state = graph_state(s, s->graphs[4 + s->p64_parity], graph_key(s, 4, s->p64_parity, SLOT_RESIDUAL, depth, p));
+    return state > 0 ? 1 : 0;
 }
 
 // Mixed-precision projection: iterative refinement of the FP64 pressure with
@@ -981,10 +1002,12 @@ static int pressure_solve_mixed(ss_sim* s, const ss_params* p, const StepConsts&
     bool conv = true;
     bool pending = false;   // the last V-cycle's correction is not in p64 yet
     bool finished = false;
-    if (tol_mode && chain_ok(s, st)) {
+    const int depth = std::min(cap, kChainDepth);
+    const int state = tol_mode ? chain_state(s, p, depth, st) : -1;
+    if (state >= 0) {
         // the first steps (all of them, as a rule) on the device; where the
         // chain ends unconverged below the cap, the host loop carries on
-        TRY(run_solve_chain(s, p, c, std::min(cap, kChainDepth), st, &done));
+        TRY(run_solve_chain(s, p, c, depth, state, st, &done));
         db = sqrt(s->red.host[SLOT_DIV_BEFORE]);
         res = sqrt(s->red.host[SLOT_RESIDUAL]);
         if (res <= mg.tol * db) {
@@ -1004,9 +1027,9 @@ static int pressure_solve_mixed(ss_sim* s, const ss_params* p, const StepConsts&
             // the last V-cycle + adding its correction and evaluating the
             // residual in one pass, recorded as one graph per buffer parity
             const int slot = stats ? SLOT_RESIDUAL : -1;
-            TRY(run_graph(s, 2 + s->p64_parity, graph_key(s, 2, s->p64_parity, slot, 1, p), st, [&]() -> int {
-                TRY(v_cycle_mixed(s, c, mg, 0, mg.precision, st));
-                return launch_ir_residual(s, c, slot, true, st);
+            TRY(run_graph(s, 2 + s->p64_parity, graph_key(s, 2, s->p64_parity, slot, 1, p), st, [&](cudaStream_t cs) -> int {
+                TRY(v_cycle_mixed(s, c, mg, 0, mg.precision, cs));
+                return launch_ir_residual(s, c, slot, true, cs);
             }));
             std::swap(s->p64, s->p64b);
             s->p64_parity ^= 1;
@@ -1045,6 +1068,7 @@ static int pressure_solve_mixed(ss_sim* s, const ss_params* p, const StepConsts&
 static int pressure_solve(ss_sim* s, const ss_params* p, const StepConsts& c, cudaStream_t st,
                           bool defer_p0 = false) {
     const ss_mg_schedule& mg = p->mg;
+    s->solves += 1;
     if (mg.precision != SS_PREC_FP32) return pressure_solve_mixed(s, p, c, st, defer_p0);
     s->p64_valid = 0;
     const bool tol_mode = mg.tol > 0.0;
@@ -1055,26 +1079,26 @@ static int pressure_solve(ss_sim* s, const ss_params* p, const StepConsts& c, cu
     int done = 0;
     bool conv = true;
     const bool rb = rb_supported(s, mg.ref_quirks);
-    auto cycle = [&]() -> int {
-        if (rb) TRY(launch_rb_convert(s, true, st));
+    auto cycle = [&](cudaStream_t cs) -> int {
+        if (rb) TRY(launch_rb_convert(s, true, cs));
         s->rb_active = rb ? 1 : 0;
-        int rc = v_cycle_rec(s, c, mg, 0, st);
+        int rc = v_cycle_rec(s, c, mg, 0, cs);
         s->rb_active = 0;
         if (rc) return rc;
-        if (rb) TRY(launch_rb_convert(s, false, st));
+        if (rb) TRY(launch_rb_convert(s, false, cs));
         return SS_OK;
     };
     if (!tol_mode) {
-        TRY(run_graph(s, 0, graph_key(s, 0, 0, stats ? SLOT_RESIDUAL : -1, rb, p), st, [&]() -> int {
-            if (rb) TRY(launch_rb_convert(s, true, st));
+        TRY(run_graph(s, 0, graph_key(s, 0, 0, stats ? SLOT_RESIDUAL : -1, rb, p), st, [&](cudaStream_t cs) -> int {
+            if (rb) TRY(launch_rb_convert(s, true, cs));
             s->rb_active = rb ? 1 : 0;
             for (int i = 0; i < cap; ++i) {
-                int rc = v_cycle_rec(s, c, mg, 0, st);
+                int rc = v_cycle_rec(s, c, mg, 0, cs);
                 if (rc) { s->rb_active = 0; return rc; }
             }
             s->rb_active = 0;
-            if (rb) TRY(launch_rb_convert(s, false, st));
-            if (stats) TRY(launch_projected_residual_norm(s, c, SLOT_RESIDUAL, st));
+            if (rb) TRY(launch_rb_convert(s, false, cs));
+            if (stats) TRY(launch_projected_residual_norm(s, c, SLOT_RESIDUAL, cs));
             return SS_OK;
         }));
         done = cap;
@@ -1089,9 +1113,9 @@ static int pressure_solve(ss_sim* s, const ss_params* p, const StepConsts& c, cu
         const double db = sqrt(s->red.host[SLOT_DIV_BEFORE]);
         double res = sqrt(s->red.host[SLOT_RESIDUAL]);
         while (done < cap && !(res <= mg.tol * db)) {
-            TRY(run_graph(s, 1, graph_key(s, 1, 0, SLOT_RESIDUAL, rb, p), st, [&]() -> int {
-                TRY(cycle());
-                return launch_projected_residual_norm(s, c, SLOT_RESIDUAL, st);
+            TRY(run_graph(s, 1, graph_key(s, 1, 0, SLOT_RESIDUAL, rb, p), st, [&](cudaStream_t cs) -> int {
+                TRY(cycle(cs));
+                return launch_projected_residual_norm(s, c, SLOT_RESIDUAL, cs);
             }));
             ++done;
             TRY(read_slots(s, st));

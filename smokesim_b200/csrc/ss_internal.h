@@ -158,16 +158,18 @@ struct ss_sim {
     struct SolveGraph {
         cudaGraphExec_t exec = nullptr;
         unsigned char key[96] = {};
+        long long seen = 0;            // the solve that first had this key (0: none)
         long long launches = 0;        // kernels of one replay (4/5: of the first residual)
         long long step_launches = 0;   // 4/5: kernels of one refinement step
     };
     SolveGraph graphs[6];
+    long long solves = 0;              // pressure solves so far
     int use_graphs = 1;
     // mixed solve to a tolerance: the first chain_depth refinement steps as
     // nested conditional graph nodes, the convergence test on the device
     // (SMOKESIM_DEVICE_LOOP=0 sets 0: a host round trip per step)
     int device_loop = 1;
-    cudaStream_t chain_stream = nullptr;   // records the nested step graphs
+    cudaStream_t record_stream = nullptr;   // records the solve graphs
     // programmatic dependent launch of the solve's kernel chain (SMOKESIM_PDL=0 sets 0)
     int pdl = 1;
     // the V-cycle's levels from coarse_from down run in one thread-block cluster
