@@ -211,24 +211,54 @@ struct RbPlane {
 // all of its own colour (+0 where the cell is not updated) and +0 over the
 // other colour (zo) - the values a clear of both arrays followed by the plain
 // half-sweep leaves.
+//
+// Bound by its instruction stream, so the quotient by the fluid-neighbour count f
+// takes the same three operations for every f: q0 = a y, r = a - f q0, q0 + r y
+// with y = RN(1/f) - div_by_count's steps, which for f = 6 halve everything by
+// an exact factor - with {f, y} from a table indexed by the mask byte.  Tiny
+// dividends, where those steps are not exact, are redone by div_by_count out of
+// line.  Threads fill warps across rows, so that short rows leave no lane idle.
+// A half-sweep in a replayed solve: 5.9 us at 128^3 (8.8 with a selected
+// reciprocal and a row of threads per grid row), 8.1 at 192x128x160 (10.4), 3.5 at
+// 64^3 (4.5; a launch's latency), 23 at 256^3 (23.5; 4.8 TB/s of the 6.5 a copy
+// reaches, part of it from L2).
+struct CountDiv {
+    float f, y;   // {0, 0}: not updated
+};
+constexpr float kRecip[7] = {0.f, 1.f, 1.f / 2.f, 1.f / 3.f, 1.f / 4.f, 1.f / 5.f, 1.f / 6.f};
+struct CountTable {
+    CountDiv e[128];
+    constexpr CountTable() : e() {
+        for (int m = 0; m < 128; ++m) {
+            int n = 0;
+            for (int b = 1; b < 7; ++b) n += (m >> b) & 1;
+            const bool upd = (m & 1) && n;
+            e[m].f = upd ? (float)n : 0.f;
+            e[m].y = upd ? kRecip[n] : 0.f;
+        }
+    }
+};
+__constant__ CountTable c_count = CountTable();
+
+__device__ __noinline__ float div_small(float a, float f) { return div_by_count(a, (int)f); }
+
 template <int DIM, bool ZERO = false, bool INIT = false>
 __global__ void __launch_bounds__(256) k_rb_smooth4(float* __restrict__ pc, const float* __restrict__ po,
                                                     const float* __restrict__ rhs_c, const uint8_t* __restrict__ mask_c,
                                                     RBLevel g, int colour, int planes, float* __restrict__ zo) {
     pdl_entry();
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    const int y = blockIdx.y * blockDim.y + threadIdx.y;
-    if (q >= (g.half >> 2) || y >= g.ny) return;
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, nq = g.half >> 2;
+    const int y = t / nq, q = t - y * nq;
+    if (y >= g.ny) return;
     const int zb = blockIdx.z * planes, ze = min(zb + planes, g.nz);
     const int xh0 = q << 2;
     const int pl = g.ny * g.half;
     const bool up = y + 1 < g.ny, dn = y > 0;
+    const bool has_l = xh0 > 0, has_r = xh0 + 4 < g.half;
     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
     // every load of a plane is issued before the first one is waited for (no
     // early exit on an all-solid quad)
-    auto load = [&](int z, RbPlane& P) {
-        const int i = (z * g.ny + y) * g.half + xh0;
-        const int par = (y + z + colour) & 1;   // x = 2*xh + par
+    auto load = [&](int z, int i, int par, RbPlane& P) {
         P.m4 = __ldg(reinterpret_cast<const uint32_t*>(mask_c + i));
         P.rhs = ldg4(rhs_c + i);
         if constexpr (INIT) return;
@@ -236,63 +266,79 @@ __global__ void __launch_bounds__(256) k_rb_smooth4(float* __restrict__ pc, cons
         P.pb = dn ? ldg4(po + i - g.half) : zero;
         P.pf = (DIM == 3 && z + 1 < g.nz) ? ldg4(po + i + pl) : zero;
         // row-end neighbour: left of the first cell (par 0) or right of the last (par 1)
-        P.extra = par == 0 ? (xh0 > 0 ? __ldg(po + i - 1) : 0.f) : (xh0 + 4 < g.half ? __ldg(po + i + 4) : 0.f);
+        P.extra = 0.f;
+        if (par ? has_r : has_l) P.extra = __ldg(po + (par ? i + 4 : i - 1));
     };
-    const int i0 = (zb * g.ny + y) * g.half + xh0;
+    int i = (zb * g.ny + y) * g.half + xh0;
+    int par = (y + zb + colour) & 1;   // x = 2*xh + par
     float4 pm = zero, pk = zero;
     RbPlane cur, nxt;
     cur.pt = cur.pb = cur.pf = zero;
     cur.extra = 0.f;
     if constexpr (!INIT) {
-        pm = ldg4(po + i0);
-        pk = (DIM == 3 && zb > 0) ? ldg4(po + i0 - pl) : zero;
+        pm = ldg4(po + i);
+        pk = (DIM == 3 && zb > 0) ? ldg4(po + i - pl) : zero;
     }
-    load(zb, cur);
+    load(zb, i, par, cur);
     nxt = cur;
-    for (int z = zb; z < ze; ++z) {
-        if (z + 1 < ze) load(z + 1, nxt);
-        const int i = (z * g.ny + y) * g.half + xh0;
-        const int par = (y + z + colour) & 1;
-        float out[4];
-        bool wr[4];
+    for (int z = zb; z < ze; ++z, i += pl, par ^= 1) {
+        if (z + 1 < ze) load(z + 1, i + pl, par ^ 1, nxt);
+        float a[4], out[4];
+        CountDiv d[4];
+        bool tiny = false;
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             const uint32_t m = (cur.m4 >> (8 * k)) & 0xFFu;
-            const int fs = __popc(m & 0x7Eu);
-            wr[k] = (m & M_FLUID) && fs != 0;
-            const float left = par ? f4(pm, k) : (k ? f4(pm, k - 1) : cur.extra);
-            const float right = par ? (k < 3 ? f4(pm, k + 1) : cur.extra) : f4(pm, k);
+            d[k] = c_count.e[m];
             float sum;
             if constexpr (INIT) {
                 sum = 0.f;
-            } else if constexpr (ZERO) {
-                sum = f4(cur.pt, k) + f4(cur.pb, k);
-                sum = sum + right;
-                sum = sum + left;
-                if constexpr (DIM == 3) {
-                    sum = sum + f4(cur.pf, k);
-                    sum = sum + f4(pk, k);
-                }
             } else {
-                sum = ((m & M_TOP) ? f4(cur.pt, k) : 0.f) + ((m & M_BOTTOM) ? f4(cur.pb, k) : 0.f);
-                sum = sum + ((m & M_RIGHT) ? right : 0.f);
-                sum = sum + ((m & M_LEFT) ? left : 0.f);
-                if constexpr (DIM == 3) {
-                    sum = sum + ((m & M_FRONT) ? f4(cur.pf, k) : 0.f);
-                    sum = sum + ((m & M_BACK) ? f4(pk, k) : 0.f);
+                const float left = par ? f4(pm, k) : (k ? f4(pm, k - 1) : cur.extra);
+                const float right = par ? (k < 3 ? f4(pm, k + 1) : cur.extra) : f4(pm, k);
+                if constexpr (ZERO) {
+                    sum = f4(cur.pt, k) + f4(cur.pb, k);
+                    sum = sum + right;
+                    sum = sum + left;
+                    if constexpr (DIM == 3) {
+                        sum = sum + f4(cur.pf, k);
+                        sum = sum + f4(pk, k);
+                    }
+                } else {
+                    sum = ((m & M_TOP) ? f4(cur.pt, k) : 0.f) + ((m & M_BOTTOM) ? f4(cur.pb, k) : 0.f);
+                    sum = sum + ((m & M_RIGHT) ? right : 0.f);
+                    sum = sum + ((m & M_LEFT) ? left : 0.f);
+                    if constexpr (DIM == 3) {
+                        sum = sum + ((m & M_FRONT) ? f4(cur.pf, k) : 0.f);
+                        sum = sum + ((m & M_BACK) ? f4(pk, k) : 0.f);
+                    }
                 }
             }
-            out[k] = wr[k] ? div_by_count(sum - f4(cur.rhs, k), fs) : 0.f;
+            a[k] = sum - f4(cur.rhs, k);
+            tiny = tiny || (fabsf(a[k]) < 7.52316385e-37f && a[k] != 0.f);
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const float q0 = __fmul_rn(a[k], d[k].y);
+            out[k] = __fmaf_rn(__fmaf_rn(-d[k].f, q0, a[k]), d[k].y, q0);
+        }
+        if (tiny) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                if (d[k].f != 0.f) out[k] = div_small(a[k], d[k].f);
         }
         if (INIT) {
+            // +0 where no update happens
+#pragma unroll
+            for (int k = 0; k < 4; ++k) out[k] = d[k].f != 0.f ? out[k] : 0.f;
             *reinterpret_cast<float4*>(pc + i) = make_float4(out[0], out[1], out[2], out[3]);
             *reinterpret_cast<float4*>(zo + i) = zero;
-        } else if (wr[0] && wr[1] && wr[2] && wr[3]) {
+        } else if (d[0].f != 0.f && d[1].f != 0.f && d[2].f != 0.f && d[3].f != 0.f) {
             *reinterpret_cast<float4*>(pc + i) = make_float4(out[0], out[1], out[2], out[3]);
         } else {
 #pragma unroll
             for (int k = 0; k < 4; ++k)
-                if (wr[k]) pc[i + k] = out[k];
+                if (d[k].f != 0.f) pc[i + k] = out[k];
         }
         pk = pm;
         pm = cur.pf;
@@ -553,7 +599,12 @@ int launch_rb_sweep(ss_sim* s, int iterations, cudaStream_t st, bool zero, bool 
     const float* rhs[2] = {s->rhs_s, s->rhs_s + h};
     const uint8_t* mask[2] = {s->rb_mask, s->rb_mask + h};
     dim3 b, gr;
-    row_launch(s->rb_vec ? g.half / 4 : g.half, g.ny, g.nz, b, gr);
+    if (s->rb_vec) {
+        b = dim3(256);
+        gr = dim3((unsigned)(((long long)(g.half / 4) * g.ny + 255) / 256), 1, g.nz);
+    } else {
+        row_launch(g.half, g.ny, g.nz, b, gr);
+    }
     // z planes per thread of the four-cell kernel: about three waves of
     // four 256-thread blocks per SM
     int planes = 1;
