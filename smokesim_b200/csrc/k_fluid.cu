@@ -8,6 +8,8 @@
 
 #include <cmath>
 
+#include <algorithm>
+
 #include "common.cuh"
 #include "ss_internal.h"
 
@@ -255,126 +257,174 @@ SS_D float yface_mean(const float* __restrict__ a, int nx, int ny, int nz, int x
     return lerp_(fetch_b(a, nx, ny, nz, x, y - 1, z, border), fetch_b(a, nx, ny, nz, x, y, z, border), 0.5f);
 }
 
+// Linear sample whose taps all lie in the array: 0 <= t < n - 1 on
+// every axis (and n below 2^22).  floor(t) is the integer part of t + 2^23
+// rounded down, so no conversion instruction is needed.
+struct Cell3 {
+    int i;              // index of the low tap
+    float wx, wy, wz;
+};
+SS_D bool tap_range(float t, float lim) { return t >= 0.f && t < lim; }
+struct TapLimits {
+    float c[3], f[3];   // upper limits of t on an axis of cells, of faces
+};
+SS_D int tap_floor(float t, float* w) {
+    const float r = __fadd_rd(t, 8388608.f);
+    *w = t - (r - 8388608.f);
+    return __float_as_int(r) - 0x4B000000;
+}
+template <int DIM>
+SS_D Cell3 taps_inside(float tx, float ty, float tz, int ax, int pl) {
+    Cell3 c;
+    const int x = tap_floor(tx, &c.wx), y = tap_floor(ty, &c.wy);
+    c.i = y * ax + x;
+    if constexpr (DIM == 3) c.i += tap_floor(tz, &c.wz) * pl;
+    return c;
+}
+template <int DIM>
+SS_D float sample_inside(const float* __restrict__ a, const Cell3& c, int ax, int pl) {
+    const float *p = a + c.i, *q = a + (c.i + ax);
+    const float c00 = __ldg(p), c10 = __ldg(p + 1), c01 = __ldg(q), c11 = __ldg(q + 1);
+    if constexpr (DIM == 2) return lerp_(lerp_(c00, c10, c.wx), lerp_(c01, c11, c.wx), c.wy);
+    const float *r = a + (c.i + pl), *s = a + (c.i + pl + ax);
+    const float d00 = __ldg(r), d10 = __ldg(r + 1), d01 = __ldg(s), d11 = __ldg(s + 1);
+    const float c0 = lerp_(lerp_(c00, c10, c.wx), lerp_(c01, c11, c.wx), c.wy);
+    const float c1 = lerp_(lerp_(d00, d10, c.wx), lerp_(d01, d11, c.wx), c.wy);
+    return lerp_(c0, c1, c.wz);
+}
+// any other point (out of line: few cells, and the branch stays short)
+template <int DIM>
+__device__ __noinline__ float sample_edge(const float* a, int ax, int ay, int az, float tx, float ty, float tz,
+                                          float border) {
+    return sample_taps<DIM>(a, ax, ay, az, make_taps<DIM>(ax, ay, az, tx, ty, tz), border);
+}
+
+// lerp(lerp(a, b, 1/2), lerp(c, d, 1/2), 1/2): halving is exact, so the same
+// value (but for operands whose quarter is subnormal, which a face position of
+// at least 1/2 absorbs when the velocity is subtracted from it)
+SS_D float mean4(float a, float b, float c, float d) {
+    return __fmaf_rn(b, 0.25f, 0.25f * a) + __fmaf_rn(d, 0.25f, 0.25f * c);
+}
+
+// One thread per cell takes the cell's low faces (and, at the high end of an
+// axis, the face past the last cell).  A face that is traced has cells on both
+// sides, so every tap of its velocity exists: the face values around the cell
+// are loaded once, before any test.  Bound by its instruction stream and the
+// latency of the gathers, which hit L1 (DRAM traffic is the 33 B a cell): six
+// blocks an SM, at the price of a few spilled words on the branch of the border
+// samples.  318 us at 256^3 (357 with clamped taps, a floor conversion and loads
+// per face; 402 at the four blocks that 62 registers allow), 73 at 160x192x144 (89).
 template <int DIM, bool BUOY>
-__global__ void __launch_bounds__(256) k_advect_velocity(FluidArgs a) {
+__global__ void __launch_bounds__(256, 6) k_advect_velocity(FluidArgs a, TapLimits lim) {
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     const int y = blockIdx.y * blockDim.y + threadIdx.y;
-    const int z = blockIdx.z * blockDim.z + threadIdx.z;
+    const int z = DIM == 3 ? blockIdx.z : 0;
     const int nx = a.nx, ny = a.ny, nz = a.nz;
+    if (x >= nx || y >= ny) return;
     const float cfl = a.c.cfl;
-    // linear indices of position (x, y, z) in the cell / w array (c), the u
-    // array and the v array, and the plane sizes: every tap of the face
-    // averages below is one of these plus a fixed offset
-    const int zy = z * ny + y;
-    const int c = zy * nx + x;
-    const int iu = c + zy, iv = c + z * nx;
     const int ux = nx + 1, pl = nx * ny, plu = ux * ny, plv = nx * (ny + 1);
-    const bool in_cell = x < nx && y < ny && z < nz;
-    // solid flags of this cell and of its -x, -y, -z neighbours (out of grid = solid)
-    const bool s_c = !in_cell || (a.flags[c] & F_SOLID);
-    // every tap of the face velocities below lies inside the arrays
-    const bool interior = x >= 1 && y >= 1 && (DIM == 2 || z >= 1) && in_cell;
-#pragma unroll
-    for (int comp = 0; comp < DIM; ++comp) {
-        const int ax = nx + (comp == 0), ay = ny + (comp == 1), az = nz + (comp == 2);
-        if (x >= ax || y >= ay || z >= az) continue;
-        const float* __restrict__ src = comp == 0 ? a.u : comp == 1 ? a.v : a.w;
-        float* __restrict__ dst = comp == 0 ? a.uo : comp == 1 ? a.vo : a.wo;
-        const int i = comp == 0 ? iu : comp == 1 ? iv : c;
-        const int id = comp == 0 ? x : comp == 1 ? y : z;
-        // the cell on the face's low side: out of grid (id == 0) counts solid
-        const bool s_lo = id == 0 || (a.flags[c - (comp == 0 ? 1 : comp == 1 ? nx : pl)] & F_SOLID);
-        float out;
-        if (id == 0 && a.c.wind[comp] != 0.f) {
-            out = a.c.wind[comp];
-        } else if (s_c || s_lo) {
-            out = 0.f;
-        } else {
-            float vel[3];
-            if (interior) {
-                // vel_at_face_interior's values, its taps addressed from i, c
-                if (comp == 0) {
-                    vel[0] = __ldg(a.u + iu);
-                    const float* pv = a.v + iv - 1;
-                    vel[1] = lerp_(lerp_(__ldg(pv), __ldg(pv + 1), 0.5f), lerp_(__ldg(pv + nx), __ldg(pv + nx + 1), 0.5f),
-                                   0.5f);
-                    if constexpr (DIM == 3) {
-                        const float* pw = a.w + c - 1;
-                        vel[2] = lerp_(lerp_(__ldg(pw), __ldg(pw + 1), 0.5f),
-                                       lerp_(__ldg(pw + pl), __ldg(pw + pl + 1), 0.5f), 0.5f);
-                    } else {
-                        vel[2] = 0.f;
-                    }
-                } else if (comp == 1) {
-                    const float* pu = a.u + iu - ux;
-                    vel[0] = lerp_(lerp_(__ldg(pu), __ldg(pu + 1), 0.5f), lerp_(__ldg(pu + ux), __ldg(pu + ux + 1), 0.5f),
-                                   0.5f);
-                    vel[1] = __ldg(a.v + iv);
-                    if constexpr (DIM == 3) {
-                        const float* pw = a.w + c - nx;
-                        vel[2] = lerp_(lerp_(__ldg(pw), __ldg(pw + nx), 0.5f),
-                                       lerp_(__ldg(pw + pl), __ldg(pw + pl + nx), 0.5f), 0.5f);
-                    } else {
-                        vel[2] = 0.f;
-                    }
-                } else {
-                    const float* pu = a.u + iu - plu;
-                    vel[0] = lerp_(lerp_(__ldg(pu), __ldg(pu + 1), 0.5f), lerp_(__ldg(pu + plu), __ldg(pu + plu + 1), 0.5f),
-                                   0.5f);
-                    const float* pv = a.v + iv - plv;
-                    vel[1] = lerp_(lerp_(__ldg(pv), __ldg(pv + nx), 0.5f), lerp_(__ldg(pv + plv), __ldg(pv + plv + nx), 0.5f),
-                                   0.5f);
-                    vel[2] = __ldg(a.w + c);
-                }
-            } else if (comp == 0) {
-                vel_at_xface<DIM>(a.u, a.v, a.w, nx, ny, nz, x, y, z, vel);
-            } else if (comp == 1) {
-                vel_at_yface<DIM>(a.u, a.v, a.w, nx, ny, nz, x, y, z, vel);
-            } else {
-                vel_at_zface(a.u, a.v, a.w, nx, ny, nz, x, y, z, vel);
-            }
-            const float gx = (float)x + (comp == 0 ? 0.f : 0.5f);
-            const float gy = (float)y + (comp == 1 ? 0.f : 0.5f);
-            const float gz = DIM == 3 ? (float)z + (comp == 2 ? 0.f : 0.5f) : 0.f;
-            const float bx = gx - vel[0] * cfl, by = gy - vel[1] * cfl, bz = gz - vel[2] * cfl;
-            const Taps t = make_taps<DIM>(ax, ay, az, bx - (comp == 0 ? 0.f : 0.5f), by - (comp == 1 ? 0.f : 0.5f),
-                                          bz - (comp == 2 ? 0.f : 0.5f));
-            out = sample_taps_fast<DIM>(src, ax, ay, az, t, 0.f);
-        }
-        if constexpr (BUOY) {
-            if (comp == 1) {
-                // the y face's two cells (out of grid = fluid)
-                const bool solid_hi = y < ny && in_cell && (a.flags[c] & F_SOLID);
-                const bool solid_lo = y > 0 && x < nx && z < nz && (a.flags[c - nx] & F_SOLID);
-                if (solid_hi || solid_lo) {
-                    out = __ldg(src + i);
-                } else {
-                    const size_t ncell = (size_t)nx * ny * nz;
-                    float total = yface_mean<DIM>(a.dens, nx, ny, nz, x, y, z, 0.f);
-                    if (a.nch == 3) {
-                        total = total + yface_mean<DIM>(a.dens + ncell, nx, ny, nz, x, y, z, 0.f);
-                        total = total + yface_mean<DIM>(a.dens + 2 * ncell, nx, ny, nz, x, y, z, 0.f);
-                    }
-                    const float T = yface_mean<DIM>(a.temp, nx, ny, nz, x, y, z, a.c.t_amb);
-                    const float buoy = -a.c.alpha * total + a.c.beta * (T - a.c.t_amb);
-                    out = out + buoy * a.c.dt;
-                }
-            }
-        }
-        dst[i] = out;
+    const int c = z * pl + y * nx + x, iu = z * plu + y * ux + x, iv = z * plv + y * nx + x;
+    // the low neighbours' offsets, 0 at the low end (those faces are not traced)
+    const int xm = x > 0 ? 1 : 0, ym = y > 0 ? 1 : 0, zm = z > 0 ? 1 : 0;
+    const float* pu = a.u + iu;
+    const float* pv = a.v + iv;
+    const float* pw = a.w + c;
+    const uint8_t fl = a.flags[c];
+    const float u0 = __ldg(pu), u1 = __ldg(pu + 1);
+    const float uy0 = __ldg(pu - ym * ux), uy1 = __ldg(pu - ym * ux + 1);
+    const float v0 = __ldg(pv), v1 = __ldg(pv + nx);
+    const float vx0 = __ldg(pv - xm), vx1 = __ldg(pv - xm + nx);
+    float uz0 = 0.f, uz1 = 0.f, vz0 = 0.f, vz1 = 0.f, w0 = 0.f, w1 = 0.f, wx0 = 0.f, wx1 = 0.f, wy0 = 0.f, wy1 = 0.f;
+    if constexpr (DIM == 3) {
+        uz0 = __ldg(pu - zm * plu), uz1 = __ldg(pu - zm * plu + 1);
+        vz0 = __ldg(pv - zm * plv), vz1 = __ldg(pv - zm * plv + nx);
+        w0 = __ldg(pw), w1 = __ldg(pw + pl);
+        wx0 = __ldg(pw - xm), wx1 = __ldg(pw - xm + pl);
+        wy0 = __ldg(pw - ym * nx), wy1 = __ldg(pw - ym * nx + pl);
     }
+    const bool solid = fl & F_SOLID;
+    const float fx = (float)x, fy = (float)y, fz = (float)z;
+    const float hx = fx + 0.5f, hy = fy + 0.5f, hz = fz + 0.5f;
+    // u face: out of grid counts solid, wind enters at the low end
+    float out = 0.f;
+    if (x == 0 && a.c.wind[0] != 0.f) {
+        out = a.c.wind[0];
+    } else if (!solid && x > 0 && !(fl & F_LEFT)) {
+        const float v = mean4(vx0, v0, vx1, v1), w = mean4(wx0, w0, wx1, w1);
+        const float tx = fx - u0 * cfl, ty = (hy - v * cfl) - 0.5f, tz = DIM == 3 ? (hz - w * cfl) - 0.5f : 0.f;
+        out = tap_range(tx, lim.f[0]) && tap_range(ty, lim.c[1]) && (DIM == 2 || tap_range(tz, lim.c[2]))
+                  ? sample_inside<DIM>(a.u, taps_inside<DIM>(tx, ty, tz, ux, plu), ux, plu)
+                  : sample_edge<DIM>(a.u, ux, ny, nz, tx, ty, tz, 0.f);
+    }
+    a.uo[iu] = out;
+    if (x == nx - 1) a.uo[iu + 1] = 0.f;
+    // v face
+    out = 0.f;
+    if (y == 0 && a.c.wind[1] != 0.f) {
+        out = a.c.wind[1];
+    } else if (!solid && y > 0 && !(fl & F_BOTTOM)) {
+        const float u = mean4(uy0, uy1, u0, u1), w = mean4(wy0, w0, wy1, w1);
+        const float tx = (hx - u * cfl) - 0.5f, ty = fy - v0 * cfl, tz = DIM == 3 ? (hz - w * cfl) - 0.5f : 0.f;
+        out = tap_range(tx, lim.c[0]) && tap_range(ty, lim.f[1]) && (DIM == 2 || tap_range(tz, lim.c[2]))
+                  ? sample_inside<DIM>(a.v, taps_inside<DIM>(tx, ty, tz, nx, plv), nx, plv)
+                  : sample_edge<DIM>(a.v, nx, ny + 1, nz, tx, ty, tz, 0.f);
+    }
+    float past = 0.f;   // the face past the last cell
+    if constexpr (BUOY) {
+        // a face touching solid (out of grid = fluid) keeps its value from before the advection
+        auto lift = [&](int yf) {
+            const size_t ncell = (size_t)nx * ny * nz;
+            float total = yface_mean<DIM>(a.dens, nx, ny, nz, x, yf, z, 0.f);
+            if (a.nch == 3) {
+                total = total + yface_mean<DIM>(a.dens + ncell, nx, ny, nz, x, yf, z, 0.f);
+                total = total + yface_mean<DIM>(a.dens + 2 * ncell, nx, ny, nz, x, yf, z, 0.f);
+            }
+            const float T = yface_mean<DIM>(a.temp, nx, ny, nz, x, yf, z, a.c.t_amb);
+            const float buoy = -a.c.alpha * total + a.c.beta * (T - a.c.t_amb);
+            return buoy * a.c.dt;
+        };
+        out = solid || (y > 0 && (fl & F_BOTTOM)) ? v0 : out + lift(y);
+        if (y == ny - 1) past = solid ? v1 : past + lift(ny);
+    }
+    a.vo[iv] = out;
+    if (y == ny - 1) a.vo[iv + nx] = past;
+    if constexpr (DIM == 3) {
+        // w face
+        out = 0.f;
+        if (z == 0 && a.c.wind[2] != 0.f) {
+            out = a.c.wind[2];
+        } else if (!solid && z > 0 && !(fl & F_BACK)) {
+            const float u = mean4(uz0, uz1, u0, u1), v = mean4(vz0, vz1, v0, v1);
+            const float tx = (hx - u * cfl) - 0.5f, ty = (hy - v * cfl) - 0.5f, tz = fz - w0 * cfl;
+            out = tap_range(tx, lim.c[0]) && tap_range(ty, lim.c[1]) && tap_range(tz, lim.f[2])
+                      ? sample_inside<3>(a.w, taps_inside<3>(tx, ty, tz, nx, pl), nx, pl)
+                      : sample_edge<3>(a.w, nx, ny, nz + 1, tx, ty, tz, 0.f);
+        }
+        a.wo[c] = out;
+        if (z == nz - 1) a.wo[c + pl] = 0.f;
+    }
+}
+
+static TapLimits tap_limits(const ss_sim* s) {
+    TapLimits lim;
+    const int n[3] = {s->nx, s->ny, s->nz};
+    for (int k = 0; k < 3; ++k) {
+        lim.c[k] = (float)std::min(n[k] - 1, 1 << 22);
+        lim.f[k] = (float)std::min(n[k], 1 << 22);
+    }
+    return lim;
 }
 
 int launch_advect_velocities(ss_sim* s, const StepConsts& c, bool fuse_buoyancy, cudaStream_t st) {
     FluidArgs a = fluid_args(s, c);
-    dim3 b(32, 8, 1);
-    dim3 g = grid_for(s->nx + 1, s->ny + 1, s->dim == 3 ? s->nz + 1 : 1, b);
+    const TapLimits lim = tap_limits(s);
+    const dim3 b(32, 8, 1), g = grid_for(s->nx, s->ny, s->dim == 3 ? s->nz : 1, b);
     if (s->dim == 3) {
-        if (fuse_buoyancy) k_advect_velocity<3, true><<<g, b, 0, st>>>(a);
-        else k_advect_velocity<3, false><<<g, b, 0, st>>>(a);
+        if (fuse_buoyancy) k_advect_velocity<3, true><<<g, b, 0, st>>>(a, lim);
+        else k_advect_velocity<3, false><<<g, b, 0, st>>>(a, lim);
     } else {
-        if (fuse_buoyancy) k_advect_velocity<2, true><<<g, b, 0, st>>>(a);
-        else k_advect_velocity<2, false><<<g, b, 0, st>>>(a);
+        if (fuse_buoyancy) k_advect_velocity<2, true><<<g, b, 0, st>>>(a, lim);
+        else k_advect_velocity<2, false><<<g, b, 0, st>>>(a, lim);
     }
     for (int d = 0; d < s->dim; ++d) s->vi[d] ^= 1;
     s->nlaunch += 1;
@@ -887,6 +937,8 @@ int launch_update_velocities_p64(ss_sim* s, const StepConsts& c, cudaStream_t st
 // advects with - the projected velocities - into the statistics slot `slot`
 // (the operator of k_divergence below, from the six faces already loaded
 // here); the last block to finish sums the blocks' partials in a fixed order.
+// Latency of the gathers bounds it: five blocks an SM, 220 us at 256^3 with DIV
+// (251 at four, 225 at six; 241 with clamped taps), 55 at 160x192x144 without (57).
 constexpr int kSmokePlanes = 4;
 SS_D double block_sum(double v);
 
@@ -898,7 +950,7 @@ struct DivFold {
 };
 
 template <int DIM, bool DIV>
-__global__ void __launch_bounds__(256) k_advect_smoke(FluidArgs a, DivFold df, int planes) {
+__global__ void __launch_bounds__(256, 5) k_advect_smoke(FluidArgs a, TapLimits lim, DivFold df, int planes) {
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     const int y = blockIdx.y * blockDim.y + threadIdx.y;
     const int nx = a.nx, ny = a.ny, nz = a.nz;
@@ -952,28 +1004,17 @@ __global__ void __launch_bounds__(256) k_advect_smoke(FluidArgs a, DivFold df, i
         const float gx = (float)x + 0.5f, gy = (float)y + 0.5f, gz = DIM == 3 ? (float)z + 0.5f : 0.f;
         const float cfl = a.c.cfl;
         const float bx = gx - vel[0] * cfl, by = gy - vel[1] * cfl, bz = gz - vel[2] * cfl;
-        const Taps t = make_taps<DIM>(nx, ny, nz, bx - 0.5f, by - 0.5f, bz - 0.5f);
-        // sample_taps_fast's values, its range test and base index formed once
-        // for every channel
-        const bool tin = t.x0 >= 0 && t.x0 + 1 < nx && t.y0 >= 0 && t.y0 + 1 < ny &&
-                         (DIM == 2 || (t.z0 >= 0 && t.z0 + 1 < nz));
-        const int tb = tin ? idx3(t.x0, t.y0, t.z0, nx, ny) : 0;
-        auto sample = [&](const float* __restrict__ f, float border) -> float {
-            if (!tin) return sample_taps<DIM>(f, nx, ny, nz, t, border);
-            const float* q = f + tb;
-            const float c00 = __ldg(q), c10 = __ldg(q + 1), c01 = __ldg(q + nx), c11 = __ldg(q + nx + 1);
-            if constexpr (DIM == 2) {
-                return lerp_(lerp_(c00, c10, t.wx), lerp_(c01, c11, t.wx), t.wy);
-            } else {
-                const float d00 = __ldg(q + pl), d10 = __ldg(q + pl + 1), d01 = __ldg(q + pl + nx),
-                            d11 = __ldg(q + pl + nx + 1);
-                const float c0 = lerp_(lerp_(c00, c10, t.wx), lerp_(c01, c11, t.wx), t.wy);
-                const float c1 = lerp_(lerp_(d00, d10, t.wx), lerp_(d01, d11, t.wx), t.wy);
-                return lerp_(c0, c1, t.wz);
-            }
-        };
-        for (int ch = 0; ch < a.nch; ++ch) a.dens_o[ch * ncell + c] = sample(a.dens + ch * ncell, 0.f);
-        a.temp_o[c] = sample(a.temp, a.c.t_amb);
+        const float tx = bx - 0.5f, ty = by - 0.5f, tz = bz - 0.5f;
+        if (tap_range(tx, lim.c[0]) && tap_range(ty, lim.c[1]) && (DIM == 2 || tap_range(tz, lim.c[2]))) {
+            const Cell3 t = taps_inside<DIM>(tx, ty, tz, nx, pl);
+            const float temp = sample_inside<DIM>(a.temp, t, nx, pl);
+            for (int ch = 0; ch < a.nch; ++ch) a.dens_o[ch * ncell + c] = sample_inside<DIM>(a.dens + ch * ncell, t, nx, pl);
+            a.temp_o[c] = temp;
+        } else {
+            for (int ch = 0; ch < a.nch; ++ch)
+                a.dens_o[ch * ncell + c] = sample_edge<DIM>(a.dens + ch * ncell, nx, ny, nz, tx, ty, tz, 0.f);
+            a.temp_o[c] = sample_edge<DIM>(a.temp, nx, ny, nz, tx, ty, tz, a.c.t_amb);
+        }
     }
     if constexpr (DIV) {
         const double bs = block_sum(acc);
@@ -1004,15 +1045,16 @@ int launch_advect_smoke(ss_sim* s, const StepConsts& c, cudaStream_t st, int div
     const int planes = z_planes((long long)((s->nx + 31) / 32) * ((s->ny + 7) / 8), s->nz,
                                 div_slot >= 0 ? 2 * kSmokePlanes : kSmokePlanes);
     dim3 g = grid_for(s->nx, s->ny, (s->nz + planes - 1) / planes, b);
+    const TapLimits lim = tap_limits(s);
     DivFold df{s->red.partial, s->red.ticket, s->red.out, div_slot};
     if (div_slot >= 0 && (int)(g.x * g.y * g.z) > s->red.max_blocks)
         return set_error(SS_E_INVALID, "reduction scratch too small");
     if (s->dim == 3) {
-        if (div_slot >= 0) k_advect_smoke<3, true><<<g, b, 0, st>>>(a, df, planes);
-        else k_advect_smoke<3, false><<<g, b, 0, st>>>(a, df, planes);
+        if (div_slot >= 0) k_advect_smoke<3, true><<<g, b, 0, st>>>(a, lim, df, planes);
+        else k_advect_smoke<3, false><<<g, b, 0, st>>>(a, lim, df, planes);
     } else {
-        if (div_slot >= 0) k_advect_smoke<2, true><<<g, b, 0, st>>>(a, df, planes);
-        else k_advect_smoke<2, false><<<g, b, 0, st>>>(a, df, planes);
+        if (div_slot >= 0) k_advect_smoke<2, true><<<g, b, 0, st>>>(a, lim, df, planes);
+        else k_advect_smoke<2, false><<<g, b, 0, st>>>(a, lim, df, planes);
     }
     s->si ^= 1;
     s->nlaunch += 1;
@@ -1061,14 +1103,15 @@ struct RhsOut {
 };
 
 // Each thread takes kDivPlanes cells up z (the face between two of them is
-// loaded once), so a block reduces up to 256 * kDivPlanes cells.
+// loaded once), so a block reduces up to 256 * kDivPlanes cells.  Five blocks
+// an SM: 149 us at 256^3 (163 with the four that 59 registers allow).
 constexpr int kDivPlanes = 8;
 
 // ep / eq (optional): the mixed solve's extrapolated warm start, elementwise
 // over the same cells (ep = 2 ep - eq in FP64, eq = the old ep), riding on this
 // pass, whose own traffic leaves HBM bandwidth to spare.
 template <int DIM>
-__global__ void __launch_bounds__(256) k_divergence(FluidArgs a, float* __restrict__ div0, float* __restrict__ div0r,
+__global__ void __launch_bounds__(256, 5) k_divergence(FluidArgs a, float* __restrict__ div0, float* __restrict__ div0r,
                                                     double* __restrict__ partial, RhsOut ro, int planes,
                                                     double* __restrict__ ep, double* __restrict__ eq) {
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
