@@ -9,6 +9,7 @@
 // division / square root, each cell rounds exactly like the CPU oracle:
 // same operation order, no contraction.
 #pragma once
+#include <algorithm>
 #include <cuda_runtime.h>
 #include <cuda_fp16.h>
 #include <cuda_bf16.h>
@@ -43,6 +44,8 @@ SS_D void pdl_entry() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
+
+SS_D void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
 SS_D float lerp_(float a, float b, float t) { return a * (1.f - t) + b * t; }
 
@@ -211,28 +214,69 @@ SS_D void vel_at_centre(const float* __restrict__ u, const float* __restrict__ v
     else out[2] = 0.f;
 }
 
-// Border sample with a branch-free interior fast path: when all taps are in
-// range one base address serves the 8 (4) loads.
-// 0 <= v && v + 1 < n, as one unsigned comparison (v is a clamped tap index)
-SS_D bool tap_pair_in(int v, int n) { return (unsigned)v < (unsigned)(n - 1); }
-
-template <int DIM>
-SS_D float sample_taps_fast(const float* __restrict__ a, int ax, int ay, int az, const Taps& t, float border) {
-    const bool in = tap_pair_in(t.x0, ax) && tap_pair_in(t.y0, ay) && (DIM == 2 || tap_pair_in(t.z0, az));
-    if (!in) return sample_taps<DIM>(a, ax, ay, az, t, border);
-    const float* p = a + idx3(t.x0, t.y0, t.z0, ax, ay);
-    const float c00 = __ldg(p), c10 = __ldg(p + 1), c01 = __ldg(p + ax), c11 = __ldg(p + ax + 1);
-    if constexpr (DIM == 2) {
-        return lerp_(lerp_(c00, c10, t.wx), lerp_(c01, c11, t.wx), t.wy);
-    } else {
-        const int pl = ax * ay;
-        const float d00 = __ldg(p + pl), d10 = __ldg(p + pl + 1), d01 = __ldg(p + pl + ax), d11 = __ldg(p + pl + ax + 1);
-        const float c0 = lerp_(lerp_(c00, c10, t.wx), lerp_(c01, c11, t.wx), t.wy);
-        const float c1 = lerp_(lerp_(d00, d10, t.wx), lerp_(d01, d11, t.wx), t.wy);
-        return lerp_(c0, c1, t.wz);
+// Linear sample whose taps all lie in the array: 0 <= t < n - 1 on
+// every axis (and n below 2^22).  floor(t) is the integer part of t + 2^23
+// rounded down, so no conversion instruction is needed.
+struct Cell3 {
+    int i;              // index of the low tap
+    float wx, wy, wz;
+};
+SS_D bool tap_range(float t, float lim) { return t >= 0.f && t < lim; }
+struct TapLimits {
+    float c[3], f[3];   // upper limits of t on an axis of cells, of faces
+};
+inline TapLimits tap_limits(const int n[3]) {
+    TapLimits lim;
+    for (int k = 0; k < 3; ++k) {
+        lim.c[k] = (float)std::min(n[k] - 1, 1 << 22);
+        lim.f[k] = (float)std::min(n[k], 1 << 22);
     }
+    return lim;
+}
+SS_D int tap_floor(float t, float* w) {
+    const float r = __fadd_rd(t, 8388608.f);
+    *w = t - (r - 8388608.f);
+    return __float_as_int(r) - 0x4B000000;
+}
+template <int DIM>
+SS_D Cell3 taps_inside(float tx, float ty, float tz, int ax, int pl) {
+    Cell3 c;
+    const int x = tap_floor(tx, &c.wx), y = tap_floor(ty, &c.wy);
+    c.i = y * ax + x;
+    if constexpr (DIM == 3) c.i += tap_floor(tz, &c.wz) * pl;
+    return c;
+}
+template <int DIM>
+SS_D float sample_inside(const float* __restrict__ a, const Cell3& c, int ax, int pl) {
+    const float *p = a + c.i, *q = a + (c.i + ax);
+    const float c00 = __ldg(p), c10 = __ldg(p + 1), c01 = __ldg(q), c11 = __ldg(q + 1);
+    if constexpr (DIM == 2) return lerp_(lerp_(c00, c10, c.wx), lerp_(c01, c11, c.wx), c.wy);
+    const float *r = a + (c.i + pl), *s = a + (c.i + pl + ax);
+    const float d00 = __ldg(r), d10 = __ldg(r + 1), d01 = __ldg(s), d11 = __ldg(s + 1);
+    const float c0 = lerp_(lerp_(c00, c10, c.wx), lerp_(c01, c11, c.wx), c.wy);
+    const float c1 = lerp_(lerp_(d00, d10, c.wx), lerp_(d01, d11, c.wx), c.wy);
+    return lerp_(c0, c1, c.wz);
+}
+// any other point (out of line: few cells, and the branch stays short)
+template <int DIM>
+__device__ __noinline__ float sample_edge(const float* a, int ax, int ay, int az, float tx, float ty, float tz,
+                                          float border) {
+    return sample_taps<DIM>(a, ax, ay, az, make_taps<DIM>(ax, ay, az, tx, ty, tz), border);
 }
 
+// a / b with y = RN(1/b) given: two residual corrections with fused
+// multiply-adds.  After the first the quotient is within one ulp, and with a
+// correctly rounded reciprocal the second then rounds it correctly (P.
+// Markstein, IBM J. Res. Dev. 34(1), 1990, theorem on the final step of a
+// quotient).  Holds while no intermediate leaves the normal numbers, and for +0
+// (a dividend within 1e-25..1e25 of a divisor near 1); elsewhere use the operator.
+SS_D float div_recip(float a, float b, float y) {
+    float q = __fmul_rn(a, y);
+    float r = __fmaf_rn(-b, q, a);
+    q = __fmaf_rn(r, y, q);
+    r = __fmaf_rn(-b, q, a);
+    return __fmaf_rn(r, y, q);
+}
 SS_D float round_half(float x) { return __half2float(__float2half_rn(x)); }
 
 // Storage types of the coarse multigrid levels: FP32, or FP16 / BF16 for the

@@ -58,19 +58,7 @@ constexpr int kThreads = 512;   // 128 registers a thread for two cells of each 
 constexpr int kCells = 2;       // cells of each colour per thread, at most
 constexpr int kMaxCtas = 16;
 
-// a / b with y = RN(1/b) given: two residual corrections with fused
-// multiply-adds.  After the first the quotient is within one ulp, and with a
-// correctly rounded reciprocal the second then rounds it correctly (P.
-// Markstein, IBM J. Res. Dev. 34(1), 1990, theorem on the final step of a
-// quotient).  Holds while no intermediate leaves the normal numbers, and for +0
-// (recip_ok); elsewhere use the operator.
-SS_D float div_recip(float a, float b, float y) {
-    float q = __fmul_rn(a, y);
-    float r = __fmaf_rn(-b, q, a);
-    q = __fmaf_rn(r, y, q);
-    r = __fmaf_rn(-b, q, a);
-    return __fmaf_rn(r, y, q);
-}
+// div_recip may take this dividend
 SS_D bool recip_ok(float a) {
     const float m = fabsf(a);
     return (m > 1e-25f && m < 1e25f) || __float_as_uint(a) == 0u;
@@ -531,7 +519,7 @@ __global__ void __launch_bounds__(kThreads) k_coarse(const __grid_constant__ Coa
     // level is at work, instead of one visit after the other.
     auto prefetch = [&](const void* p, long long bytes) {
         for (long long i = ((long long)rank * kThreads + threadIdx.x) * 128; i < bytes; i += (long long)ctas * kThreads * 128)
-            asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const char*>(p) + i));
+            prefetch_l2(reinterpret_cast<const char*>(p) + i);
     };
     for (int l = 1; l < b.nlev; ++l) prefetch(b.alpha[l], 4LL * b.lv[l].n[0] * b.lv[l].n[1] * b.lv[l].n[2]);
     if (b.cmat) {

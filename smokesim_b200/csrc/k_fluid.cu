@@ -257,48 +257,6 @@ SS_D float yface_mean(const float* __restrict__ a, int nx, int ny, int nz, int x
     return lerp_(fetch_b(a, nx, ny, nz, x, y - 1, z, border), fetch_b(a, nx, ny, nz, x, y, z, border), 0.5f);
 }
 
-// Linear sample whose taps all lie in the array: 0 <= t < n - 1 on
-// every axis (and n below 2^22).  floor(t) is the integer part of t + 2^23
-// rounded down, so no conversion instruction is needed.
-struct Cell3 {
-    int i;              // index of the low tap
-    float wx, wy, wz;
-};
-SS_D bool tap_range(float t, float lim) { return t >= 0.f && t < lim; }
-struct TapLimits {
-    float c[3], f[3];   // upper limits of t on an axis of cells, of faces
-};
-SS_D int tap_floor(float t, float* w) {
-    const float r = __fadd_rd(t, 8388608.f);
-    *w = t - (r - 8388608.f);
-    return __float_as_int(r) - 0x4B000000;
-}
-template <int DIM>
-SS_D Cell3 taps_inside(float tx, float ty, float tz, int ax, int pl) {
-    Cell3 c;
-    const int x = tap_floor(tx, &c.wx), y = tap_floor(ty, &c.wy);
-    c.i = y * ax + x;
-    if constexpr (DIM == 3) c.i += tap_floor(tz, &c.wz) * pl;
-    return c;
-}
-template <int DIM>
-SS_D float sample_inside(const float* __restrict__ a, const Cell3& c, int ax, int pl) {
-    const float *p = a + c.i, *q = a + (c.i + ax);
-    const float c00 = __ldg(p), c10 = __ldg(p + 1), c01 = __ldg(q), c11 = __ldg(q + 1);
-    if constexpr (DIM == 2) return lerp_(lerp_(c00, c10, c.wx), lerp_(c01, c11, c.wx), c.wy);
-    const float *r = a + (c.i + pl), *s = a + (c.i + pl + ax);
-    const float d00 = __ldg(r), d10 = __ldg(r + 1), d01 = __ldg(s), d11 = __ldg(s + 1);
-    const float c0 = lerp_(lerp_(c00, c10, c.wx), lerp_(c01, c11, c.wx), c.wy);
-    const float c1 = lerp_(lerp_(d00, d10, c.wx), lerp_(d01, d11, c.wx), c.wy);
-    return lerp_(c0, c1, c.wz);
-}
-// any other point (out of line: few cells, and the branch stays short)
-template <int DIM>
-__device__ __noinline__ float sample_edge(const float* a, int ax, int ay, int az, float tx, float ty, float tz,
-                                          float border) {
-    return sample_taps<DIM>(a, ax, ay, az, make_taps<DIM>(ax, ay, az, tx, ty, tz), border);
-}
-
 // lerp(lerp(a, b, 1/2), lerp(c, d, 1/2), 1/2): halving is exact, so the same
 // value (but for operands whose quarter is subnormal, which a face position of
 // at least 1/2 absorbs when the velocity is subtracted from it)
@@ -405,19 +363,9 @@ __global__ void __launch_bounds__(256, 6) k_advect_velocity(FluidArgs a, TapLimi
     }
 }
 
-static TapLimits tap_limits(const ss_sim* s) {
-    TapLimits lim;
-    const int n[3] = {s->nx, s->ny, s->nz};
-    for (int k = 0; k < 3; ++k) {
-        lim.c[k] = (float)std::min(n[k] - 1, 1 << 22);
-        lim.f[k] = (float)std::min(n[k], 1 << 22);
-    }
-    return lim;
-}
-
 int launch_advect_velocities(ss_sim* s, const StepConsts& c, bool fuse_buoyancy, cudaStream_t st) {
     FluidArgs a = fluid_args(s, c);
-    const TapLimits lim = tap_limits(s);
+    const TapLimits lim = tap_limits(s->lv[0].n);
     const dim3 b(32, 8, 1), g = grid_for(s->nx, s->ny, s->dim == 3 ? s->nz : 1, b);
     if (s->dim == 3) {
         if (fuse_buoyancy) k_advect_velocity<3, true><<<g, b, 0, st>>>(a, lim);
@@ -1045,7 +993,7 @@ int launch_advect_smoke(ss_sim* s, const StepConsts& c, cudaStream_t st, int div
     const int planes = z_planes((long long)((s->nx + 31) / 32) * ((s->ny + 7) / 8), s->nz,
                                 div_slot >= 0 ? 2 * kSmokePlanes : kSmokePlanes);
     dim3 g = grid_for(s->nx, s->ny, (s->nz + planes - 1) / planes, b);
-    const TapLimits lim = tap_limits(s);
+    const TapLimits lim = tap_limits(s->lv[0].n);
     DivFold df{s->red.partial, s->red.ticket, s->red.out, div_slot};
     if (div_slot >= 0 && (int)(g.x * g.y * g.z) > s->red.max_blocks)
         return set_error(SS_E_INVALID, "reduction scratch too small");

@@ -35,26 +35,89 @@ struct RenderArgs {
     float kd, ks, step, shadow_step;
     int shadow_steps;
     float g;
-    float box[3];
+    float box[3], rbox[3], n[3];   // rbox = RN(1 / box), n: cells
+    TapLimits lim;
 };
 
 SS_D float fract_(float x) { return x - floorf(x); }
 
-// smoke rgb at a box-space point (single channel: grey)
-SS_D void smoke_rgb(const RenderArgs& a, float px, float py, float pz, float rgb[3]) {
-    const float tx = (px / a.box[0]) * (float)a.nx - 0.5f;
-    const float ty = (py / a.box[1]) * (float)a.ny - 0.5f;
-    const float tz = (pz / a.box[2]) * (float)a.nz - 0.5f;
-    const Taps t = make_taps<3>(a.nx, a.ny, a.nz, tx, ty, tz);
+// texel-space coordinates of a box-space point.  The quotient is exact but where
+// it is so small that it vanishes against 1/2 either way.
+SS_D bool texel(const RenderArgs& a, const float p[3], float t[3]) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) t[k] = div_recip(p[k], a.box[k], a.rbox[k]) * a.n[k] - 0.5f;
+    return tap_range(t[0], a.lim.c[0]) && tap_range(t[1], a.lim.c[1]) && tap_range(t[2], a.lim.c[2]);
+}
+
+// smoke rgb at texel-space coordinates (single channel: grey), all taps in the grid
+template <int NCH>
+SS_D void smoke_inside(const RenderArgs& a, const Cell3& c, float rgb[3]) {
+    const int pl = a.nx * a.ny;
+    const size_t n = (size_t)pl * a.nz;
+    rgb[0] = sample_inside<3>(a.dens, c, a.nx, pl);
+    rgb[1] = NCH == 3 ? sample_inside<3>(a.dens + n, c, a.nx, pl) : rgb[0];
+    rgb[2] = NCH == 3 ? sample_inside<3>(a.dens + 2 * n, c, a.nx, pl) : rgb[0];
+}
+
+// the same at any other point
+template <int NCH>
+SS_D void smoke_edge(const RenderArgs& a, const float t[3], float rgb[3]) {
+    rgb[0] = rgb[1] = rgb[2] = 0.f;
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+        if (t[k] < -1.f || t[k] >= a.n[k]) return;   // no tap in the grid
     const size_t n = (size_t)a.nx * a.ny * a.nz;
-    rgb[0] = sample_taps_fast<3>(a.dens, a.nx, a.ny, a.nz, t, 0.f);
-    if (a.nch == 3) {
-        rgb[1] = sample_taps_fast<3>(a.dens + n, a.nx, a.ny, a.nz, t, 0.f);
-        rgb[2] = sample_taps_fast<3>(a.dens + 2 * n, a.nx, a.ny, a.nz, t, 0.f);
-    } else {
-        rgb[1] = rgb[0];
-        rgb[2] = rgb[0];
+    rgb[0] = sample_edge<3>(a.dens, a.nx, a.ny, a.nz, t[0], t[1], t[2], 0.f);
+    rgb[1] = NCH == 3 ? sample_edge<3>(a.dens + n, a.nx, a.ny, a.nz, t[0], t[1], t[2], 0.f) : rgb[0];
+    rgb[2] = NCH == 3 ? sample_edge<3>(a.dens + 2 * n, a.nx, a.ny, a.nz, t[0], t[1], t[2], 0.f) : rgb[0];
+}
+
+// Density between a point of the ray and the light.  Two samples at a time, their
+// loads in flight together (three: 260 us, six: 30 more); the march ends early once it has left
+// the box for good (every further sample is zero).
+constexpr int kShadowBatch = 2;
+template <int NCH>
+SS_D float shadow(const RenderArgs& a, const float pos[3]) {
+    float lp[3] = {pos[0], pos[1], pos[2]};
+    float ld = 0.f;
+    for (int j = 0; j < a.shadow_steps; j += kShadowBatch) {
+        float t[kShadowBatch][3], total[kShadowBatch];
+        bool in[kShadowBatch];
+#pragma unroll
+        for (int u = 0; u < kShadowBatch; ++u) {
+#pragma unroll
+            for (int k = 0; k < 3; ++k) lp[k] = lp[k] + a.light[k] * a.shadow_step;
+            in[u] = texel(a, lp, t[u]);
+        }
+#pragma unroll
+        for (int u = 0; u < kShadowBatch; ++u) {
+            Cell3 c;
+            const int x = tap_floor(in[u] ? t[u][0] : 0.f, &c.wx), y = tap_floor(in[u] ? t[u][1] : 0.f, &c.wy),
+                      z = tap_floor(in[u] ? t[u][2] : 0.f, &c.wz);
+            c.i = (z * a.ny + y) * a.nx + x;
+            float s[3];
+            smoke_inside<NCH>(a, c, s);
+            total[u] = s[0] + s[1] + s[2];
+        }
+        bool gone = false;
+#pragma unroll
+        for (int u = 0; u < kShadowBatch; ++u) {
+            if (j + u >= a.shadow_steps) break;
+            if (!in[u]) {
+                float s[3];
+                smoke_edge<NCH>(a, t[u], s);
+                total[u] = s[0] + s[1] + s[2];
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    const float d = a.light[k] * a.shadow_step;
+                    gone = gone || (d > 0.f && t[u][k] >= a.n[k]) || (d < 0.f && t[u][k] < -1.f);
+                }
+            }
+            ld = ld + total[u];
+        }
+        if (gone) break;
     }
+    return ld;
 }
 
 SS_D unsigned char to_unorm8(float v) {
@@ -62,9 +125,20 @@ SS_D unsigned char to_unorm8(float v) {
     return (unsigned char)(v * 255.f + 0.5f);
 }
 
-__global__ void __launch_bounds__(256) k_raymarch(RenderArgs a, uchar4* __restrict__ out) {
-    const int px = blockIdx.x * blockDim.x + threadIdx.x;
-    const int row = blockIdx.y * blockDim.y + threadIdx.y;
+// i-th of n places from the middle outwards
+SS_D int centre_out(int i, int n) { return (n - 1) / 2 + ((i & 1) ? (i + 1) / 2 : -(i / 2)); }
+
+// A warp takes 8 x 4 pixels, whose rays stay together, and a block four warps, so
+// that a long ray holds few others' place; blocks go from the middle of the
+// picture, where the smoke is, outwards, so that the last ones end soon.  Bound by
+// its instructions: 234 us for 1024 x 1024 rays through 192^3 cells of dense smoke;
+// 464 with rows of 32 pixels in blocks of 256, one shadow sample at a time, IEEE
+// divisions and clamped taps (248e6 warp instructions against 177e6; 272 with rows
+// from the top).
+template <int NCH>
+__global__ void __launch_bounds__(128) k_raymarch(RenderArgs a, uchar4* __restrict__ out) {
+    const int px = centre_out(blockIdx.x, gridDim.x) * 8 + (threadIdx.x & 7);
+    const int row = centre_out(blockIdx.y, gridDim.y) * 16 + (threadIdx.x >> 3);
     if (px >= a.W || row >= a.H) return;
     const int py = a.H - 1 - row;   // the shader's gl_FragCoord.y runs upwards
     const float u = ((float)px + 0.5f) / (float)a.W, v = ((float)py + 0.5f) / (float)a.H;
@@ -107,19 +181,12 @@ __global__ void __launch_bounds__(256) k_raymarch(RenderArgs a, uchar4* __restri
     for (int i = 0; i < steps; ++i) {
         if (t > exit_) break;
         const float pos[3] = {a.cam[0] + dir[0] * t, a.cam[1] + dir[1] * t, a.cam[2] + dir[2] * t};
-        float rgb[3];
-        smoke_rgb(a, pos[0], pos[1], pos[2], rgb);
+        float rgb[3], tx[3];
+        if (texel(a, pos, tx)) smoke_inside<NCH>(a, taps_inside<3>(tx[0], tx[1], tx[2], a.nx, a.nx * a.ny), rgb);
+        else smoke_edge<NCH>(a, tx, rgb);
         const float total = rgb[0] + rgb[1] + rgb[2];
         if (total > 0.001f) {
-            float ld = 0.f;
-            float lp[3] = {pos[0], pos[1], pos[2]};
-            for (int j = 0; j < a.shadow_steps; ++j) {
-#pragma unroll
-                for (int k = 0; k < 3; ++k) lp[k] = lp[k] + a.light[k] * a.shadow_step;
-                float s[3];
-                smoke_rgb(a, lp[0], lp[1], lp[2], s);
-                ld = ld + (s[0] + s[1] + s[2]);
-            }
+            const float ld = shadow<NCH>(a, pos);
             const float atten = expf(-ld * a.ks * a.shadow_step);
             const float alpha = 1.f - expf(-total * a.kd * a.step);
             const float ta = T * alpha;
@@ -256,8 +323,18 @@ int ss_render(ss_sim* s, const ss_render_desc* d, uint8_t* rgba, int on_device, 
         dst = (uchar4*)s->render_buf;
     }
     dim3 b(32, 8, 1), g((d->width + 31) / 32, (d->height + 7) / 8, 1);
-    if (s->dim == 3) k_raymarch<<<g, b, 0, st>>>(a, dst);
-    else k_draw2d<<<g, b, 0, st>>>(a, dst);
+    if (s->dim == 3) {
+        a.lim = tap_limits(s->lv[0].n);
+        for (int k = 0; k < 3; ++k) {
+            a.n[k] = (float)s->lv[0].n[k];
+            a.rbox[k] = 1.f / a.box[k];
+        }
+        const dim3 gr((d->width + 7) / 8, (d->height + 15) / 16);
+        if (s->nch == 3) k_raymarch<3><<<gr, 128, 0, st>>>(a, dst);
+        else k_raymarch<1><<<gr, 128, 0, st>>>(a, dst);
+    } else {
+        k_draw2d<<<g, b, 0, st>>>(a, dst);
+    }
     int rc = check_cuda(cudaGetLastError(), "render");
     if (rc) return rc;
     if (!on_device) {
