@@ -67,12 +67,15 @@ __global__ void k_f32_from_p64(const double* __restrict__ p64, float* __restrict
 // (p_in and p_out are different buffers - neighbours read p_in + e).  Each
 // block takes kIrChunk z planes of a 32x8 column, so a block reduces up to
 // 256 * kIrChunk cells.
+// Bound by the memory latency that four blocks an SM can hide: 126 us with the
+// correction at 256^3 (553 MB, 4.4 TB/s), 94 without; 20.2 and 18.4 at 128^3.
 // A block owns a 32x8 column of cells and marches up kIrChunk z planes.  The
 // pressure after the pending correction, P = p_in + e, is evaluated once per
 // cell: the column's own values roll through registers (the z neighbours),
 // each plane's tile plus its one-cell x/y rim goes through shared memory (the
 // x and y neighbours), double-buffered so a plane costs one barrier.
-constexpr int kIrTX = 32, kIrTY = 8, kIrChunk = 16;   // largest z chunk
+constexpr int kIrTX = 32, kIrTY = 8, kIrChunk = 32;   // largest z chunk
+constexpr int kIrAhead = 4;
 constexpr int kIrRim = 2 * kIrTX + 2 * kIrTY;   // rim cells of a tile (no corners: 5/7-point stencil)
 
 // DEC: the launch carries the device-side convergence test (IrDecide) of the
@@ -85,7 +88,7 @@ __global__ void __launch_bounds__(kIrTX * kIrTY) k_ir_residual(
     const float* __restrict__ div0, const uint8_t* __restrict__ fmask, int nx, int ny, int nz, double k,
     double inv_k, double inv_khh, float* __restrict__ rhs_s, float* __restrict__ rhs_r, double* __restrict__ psum,
     double* __restrict__ pmax, unsigned int* __restrict__ ticket, double* __restrict__ out, int slot,
-    float* __restrict__ scale, int planes, IrDecide dec) {
+    float* __restrict__ scale, int planes, int prefetch, IrDecide dec) {
     pdl_entry();
     __shared__ double sP[2][kIrTY + 2][kIrTX + 2];
     const int tx = threadIdx.x, ty = threadIdx.y, tid = tx + kIrTX * ty;
@@ -143,8 +146,33 @@ __global__ void __launch_bounds__(kIrTX * kIrTY) k_ir_residual(
     };
     Ahead qa;
     fetch(zb + 1, qa);
+    // with `prefetch` a warp also brings its row's lines of the arrays into L2,
+    // one line per lane, kIrAhead planes before they are read
+    const char* pf = nullptr;
+    size_t pf_step = 0;
+    if (prefetch && y < ny) {
+        const int row = idx3(x0, y, zb, nx, ny), pl = nx * ny;
+        if (tx == 0 || (tx == 1 && x0 + 16 < nx)) {
+            pf = reinterpret_cast<const char*>(p_in + row + 16 * tx);
+            pf_step = sizeof(double) * pl;
+        } else if (tx == 2) {
+            pf = reinterpret_cast<const char*>(div0 + row);
+            pf_step = sizeof(float) * pl;
+        } else if (tx == 3) {
+            pf = reinterpret_cast<const char*>(fmask + row);
+            pf_step = pl;
+        } else if (ACC && (tx == 4 || tx == 5)) {
+            pf = reinterpret_cast<const char*>(e + (tx == 5 ? (pl >> 1) * nz : 0) + (row >> 1));
+            pf_step = sizeof(float) * (pl >> 1);
+        }
+        if (pf) pf += kIrAhead * pf_step;
+    }
     for (int z = zb; z < ze; ++z) {
         const int sl = z & 1;
+        if (pf) {
+            if (z + kIrAhead < min(ze + 1, nz)) prefetch_l2(pf);
+            pf += pf_step;
+        }
         sP[sl][ty + 1][tx + 1] = p0;
         if (tid < kIrRim) sP[sl][hy][hx] = h0;
         Ahead qb;
@@ -281,7 +309,12 @@ int launch_ir_residual(ss_sim* s, const StepConsts& c, int slot, bool accumulate
     if (d.active && slot != SLOT_RESIDUAL) return set_error(SS_E_INVALID, "the convergence test reads the residual slot");
     dim3 b(kIrTX, kIrTY, 1);
     const int tx = (s->nx + kIrTX - 1) / kIrTX, ty = (s->ny + kIrTY - 1) / kIrTY;
-    const int planes = z_planes((long long)tx * ty, s->nz, kIrChunk);
+    // one wave of the four blocks an SM holds, so that the fewest planes are loaded
+    // twice: 20.2 us with the correction at 128^3 (22.5 in two waves)
+    const int planes = z_planes((long long)tx * ty, s->nz, kIrChunk, 1, 148LL * 4);
+    // where the arrays do not stay in the 126 MB of L2: 125 us against 134 at 256^3
+    // (285 MB); at 128^3 (36 MB) its instructions cost 1.6 us of 22.5
+    const int prefetch = (long long)s->ncell * 17 > 96LL << 20;
     dim3 g(tx, ty, (s->nz + planes - 1) / planes);
     const int nblocks = (int)(g.x * g.y * g.z);
     if (nblocks > s->red.max_blocks) return set_error(SS_E_INVALID, "reduction scratch too small");
@@ -294,7 +327,7 @@ int launch_ir_residual(ss_sim* s, const StepConsts& c, int slot, bool accumulate
     float* rhs_r = s->rhs_r_is_s ? nullptr : s->rhs_r;
 #define IR_ARGS(ACC) s->p64, s->p_alt, s->p64b, s->div0, s->fmask, s->nx, s->ny, s->nz, k, inv_k, inv_khh, \
                      s->rhs_s, rhs_r, s->red.partial, s->red.partial_max, s->red.ticket, s->red.out, slot, \
-                     s->d_scale, planes, d
+                     s->d_scale, planes, prefetch, d
     if (s->dim == 3) {
         if (d.active) {
             if (accumulate) launch_k(s->pdl, g, b, 0, st, k_ir_residual<3, true, true>, IR_ARGS(true));

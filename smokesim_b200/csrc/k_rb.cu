@@ -349,8 +349,10 @@ __global__ void __launch_bounds__(256) k_rb_smooth4(float* __restrict__ pc, cons
 // Residual of the fine cells under four consecutive coarse cells of a row,
 // restricted: per fine row the even-x cells sit in one colour array and the
 // odd-x cells in the other, both at the coarse x index.
+// Four blocks an SM, a few words spilled: 42.5 us at 256^3 (46.3 at three, 52.5 at
+// five), 9.1 at 128^3 in the mixed solve (10.6, 11.7).
 template <int DIM, bool POW2, typename T = float, bool ZERO = false>
-__global__ void __launch_bounds__(256, 3) k_rb_residual_restrict4(const float* __restrict__ p_red, const float* __restrict__ p_black,
+__global__ void __launch_bounds__(256, 4) k_rb_residual_restrict4(const float* __restrict__ p_red, const float* __restrict__ p_black,
                                                                const float* __restrict__ rr_red, const float* __restrict__ rr_black,
                                                                const uint8_t* __restrict__ m_red, const uint8_t* __restrict__ m_black,
                                                                RBLevel g, T* __restrict__ rc, int cx, int cy,
