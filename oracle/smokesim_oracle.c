@@ -919,7 +919,7 @@ void og_prolong_and_add(og_sim* s, int L) {
  * as the pre-smoother, and both operators use one out-of-grid rule. */
 /* The mixed solve's coarsest level (levels >= 2, at most 1024 cells) is not
  * swept: its n_coarse red-black iterations from p = 0 are a linear map of the
- * right-hand side, applied as a matrix (k_mg.cu k_bottom / coarse_product).
+ * right-hand side, applied as a matrix (coarse_level.cuh coarse_product).
  * The matrix is the iterations' response to unit right-hand sides in FP32
  * without the coarse-storage rounding, rebuilt when the level's solid
  * fractions or the iteration count change; p_j = cstore(sum_i cm[i n + j] r_i)

@@ -391,7 +391,7 @@ int ss_adjoint_create(ss_sim* s, int nsteps, int every, ss_adjoint** out) {
     }
     W((void**)&A->fpart, (size_t)adj_force_blocks(s) * 3 * sizeof(double));
     W((void**)&A->fgrad, (size_t)nsteps * 3 * sizeof(double));
-    // the bottom solve's adjoint applies the coarsest sweeps as one matrix
+    // the lower V-cycle's transpose applies the coarsest sweeps as one matrix
     // (SMOKESIM_ADJ_COARSE_SWEEPS=1 transposes them sweep by sweep instead)
     {
         const ss::Level& lc = s->lv[s->levels - 1];
@@ -399,6 +399,7 @@ int ss_adjoint_create(ss_sim* s, int nsteps, int every, ss_adjoint** out) {
         const char* e = getenv("SMOKESIM_ADJ_COARSE_SWEEPS");
         if (s->levels >= 2 && nc <= kCoarseResponseMax && !(e && atoi(e) != 0)) {
             W((void**)&A->cresp, (size_t)(nc * nc) * 4);
+            W((void**)&A->w.cpart, kProductLanes * 4);
             A->cresp_n = (int)nc;
         }
     }

@@ -237,7 +237,6 @@ int ss_create(const ss_desc* d, void* stream, ss_sim** out) {
         s->lv[l].h = s->h * (float)(1 << l);
         s->lv[l].hh = s->lv[l].h * s->lv[l].h;
     }
-    s->bottom = bottom_start(s);
 
     int rc = coarse_setup(s);
     auto A = [&](void** p, size_t bytes) { if (rc == SS_OK) rc = dalloc(p, bytes); };

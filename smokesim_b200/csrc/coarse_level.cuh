@@ -48,7 +48,7 @@ SS_D float ldv(const T* p) {
 // cells and cells without fluid neighbours are skipped; out of grid = fluid
 // with p = 0.
 // R: the type whose rounding every stored pressure gets (== T for global
-// arrays; the shared-memory bottom solve keeps float storage rounded as R).
+// arrays).
 template <int DIM, bool L0, typename T = float, typename R = T, bool CG = false>
 SS_D void smooth_cell(const MGArgsT<T>& a, int x, int y, int z) {
     const int nx = a.nx, ny = a.ny, nz = a.nz;
@@ -203,8 +203,7 @@ SS_D float residual_cell(const MGArgsT<T>& a, int x, int y, int z) {
 // ((i - i0) mod 8), added pairwise, so the oracle can repeat the order.  Two
 // rounds of eight independent loads are in flight per step (the matrix
 // streams from L2).
-// r: the level's right-hand side (shared-memory floats in the one-block
-// bottom solve, the level's global array with CG in the cluster form).
+// r: the level's right-hand side, in shared memory or (CG) global.
 template <bool CG = false, typename RT>
 SS_D float coarse_product(const float* __restrict__ E, const RT* r, int n, int j, int i0, int i1) {
     float a[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
@@ -224,10 +223,9 @@ SS_D float coarse_product(const float* __restrict__ E, const RT* r, int n, int j
 }
 
 // Slices of i per coarse value in the matrix product: the largest power of
-// two (at most 32) with parts * n <= kProductLanes, a cluster's threads - so
-// the cluster form takes one slice (at most 16 terms at 8^3) per thread.  The
-// one-block bottom solve walks the same (slice, value) items in turns of its
-// 1024 threads, so both give the same sums in the same order.
+// two (at most 32) with parts * n <= kProductLanes, twice the threads of the
+// largest cluster - slices of at most 16 terms at 8^3.  The number depends on n
+// alone, so every cluster size gives the same sums in the same order.
 SS_D int coarse_parts(int n) {
     int parts = 1;
     while (parts < 32 && parts * 2 * n <= kProductLanes) parts *= 2;

@@ -1271,322 +1271,13 @@ static int adj_sweeps(ss_sim* s, const AdjLevel& a, int L, int iterations, cudaS
     return check_cuda(cudaGetLastError(), "k_adj_smooth");
 }
 
-// ------------------------------------------------ single-block lower V-cycle^T
-// The transpose of the lower V-cycle: levels Lb..coarsest in one thread block with the
-// adjoint arrays (pbar, bbar, T of every level) in shared memory - the
-// 2*n_coarse + 1 launches of the coarsest level's transposed sweeps alone
-// would otherwise dominate.  Same per-cell operations as the level kernels
-// above, one __syncthreads per half-step.
-struct AdjBottomArgs {
-    int nlev;
-    int n[SS_MAX_LEVELS][3];
-    int off[SS_MAX_LEVELS];
-    float hh[SS_MAX_LEVELS];
-    const float* alpha[SS_MAX_LEVELS];
-    float* pbar0;   // global adjoint pressure of level Lb (in/out)
-    float* bbar0;   // global right-hand-side adjoint of level Lb (accumulated)
-    int total;
-    int n_pre, n_post, n_coarse;
-    float oobA;
-    const float* cresp;   // coarsest level's response matrix, or null
-};
-
-SS_D AdjLevel bottom_adj_level(const AdjBottomArgs& b, int l, float* sp, float* sb, float* sT) {
-    AdjLevel a;
-    a.nx = b.n[l][0]; a.ny = b.n[l][1]; a.nz = b.n[l][2];
-    a.fmask = nullptr;
-    a.alpha = b.alpha[l];
-    a.oobA = b.oobA;
-    a.hh = b.hh[l];
-    a.beta = b.hh[l];
-    a.rcoef = 1.f;
-    a.pbar = sp + b.off[l];
-    a.bbar = sb + b.off[l];
-    a.T = sT + b.off[l];
-    return a;
-}
-
-template <int DIM>
-SS_D void bottom_adj_half(const AdjLevel& a, int colour, bool do_b, bool do_a) {
-    const int n = a.nx * a.ny * a.nz;
-    for (int q = threadIdx.x; q < n; q += blockDim.x) {
-        const int x = q % a.nx, t = q / a.nx, y = t % a.ny, z = t / a.ny;
-        if (((x + y + z) & 1) != colour) continue;
-        float wself, d;
-        bool fluid;
-        cell_weights<DIM, false>(a, x, y, z, wself, d, fluid);
-        float pb = a.pbar[q];
-        if (do_b) pb += wself * nbr_sum<DIM>(a.T, x, y, z, a.nx, a.ny, a.nz);
-        if (do_a) {
-            if (fluid && d != 0.f) {
-                const float tt = pb / d;
-                a.T[q] = tt;
-                pb = 0.f;
-                a.bbar[q] -= a.beta * tt;
-            } else {
-                a.T[q] = 0.f;
-            }
-        }
-        a.pbar[q] = pb;
-    }
-    __syncthreads();
-}
-
-// A level of at most two cells per active thread (the coarsest one): the
-// cells' weights and neighbour masks stay in registers for all the sweeps.
-template <int DIM, int CELLS>
-SS_D void bottom_adj_sweeps_cached(const AdjLevel& a, int iterations, int nt) {
-    const int n = a.nx * a.ny * a.nz;
-    const int nx = a.nx, ny = a.ny, pl = nx * ny;
-    // per cell: bits 0-5 neighbour in grid (+y,-y,+x,-x,+z,-z), 6 colour,
-    // 7 present, 8 updated by the forward smoother
-    int fl[CELLS];
-    float ws[CELLS], dd[CELLS];
-#pragma unroll
-    for (int k = 0; k < CELLS; ++k) {
-        const int c = threadIdx.x + k * nt;
-        fl[k] = 0; ws[k] = 0.f; dd[k] = 1.f;
-        if (c >= n) continue;
-        const int x = c % nx, t = c / nx, y = t % ny, z = t / ny;
-        bool fluid;
-        cell_weights<DIM, false>(a, x, y, z, ws[k], dd[k], fluid);
-        fl[k] = (y + 1 < ny ? 1 : 0) | (y > 0 ? 2 : 0) | (x + 1 < nx ? 4 : 0) | (x > 0 ? 8 : 0) |
-                (z + 1 < a.nz ? 16 : 0) | (z > 0 ? 32 : 0) | (((x + y + z) & 1) << 6) | 128 |
-                ((fluid && dd[k] != 0.f) ? 256 : 0);
-    }
-    auto half = [&](int colour, bool do_b, bool do_a) {
-#pragma unroll
-        for (int k = 0; k < CELLS; ++k) {
-            const int m = fl[k];
-            if (!(m & 128) || ((m >> 6) & 1) != colour) continue;
-            const int c = threadIdx.x + k * nt;
-            float pb = a.pbar[c];
-            if (do_b) {
-                float sum = 0.f;
-                if (m & 1) sum += a.T[c + nx];
-                if (m & 2) sum += a.T[c - nx];
-                if (m & 4) sum += a.T[c + 1];
-                if (m & 8) sum += a.T[c - 1];
-                if (DIM == 3 && (m & 16)) sum += a.T[c + pl];
-                if (DIM == 3 && (m & 32)) sum += a.T[c - pl];
-                pb += ws[k] * sum;
-            }
-            if (do_a) {
-                if (m & 256) {
-                    const float tt = pb / dd[k];
-                    a.T[c] = tt;
-                    pb = 0.f;
-                    a.bbar[c] -= a.beta * tt;
-                } else {
-                    a.T[c] = 0.f;
-                }
-            }
-            a.pbar[c] = pb;
-        }
-        if (nt == (int)blockDim.x) __syncthreads();
-        else asm volatile("bar.sync 1, %0;" ::"r"(nt) : "memory");
-    };
-    // half-steps h = 0..2*iterations: colour 1, 0, 1, ..., the first without
-    // the gather, the last without the update (one call site keeps the code small)
-    for (int h = 0; h <= 2 * iterations; ++h) half((h & 1) ? 0 : 1, h > 0, h < 2 * iterations);
-}
-
-template <int DIM>
-SS_D void bottom_adj_sweeps(const AdjLevel& a, int iterations) {
-    if (iterations <= 0) return;
-    const int n = a.nx * a.ny * a.nz;
-    int nt = blockDim.x;
-    // the fewest threads that still give every cell its own thread (the
-    // coarsest 8^3 level: 512); measured faster than two cells a thread
-    while (nt > 128 && (n + nt / 2 - 1) / (nt / 2) <= 1) nt /= 2;
-    if ((n + nt - 1) / nt <= 2) {
-        if ((int)threadIdx.x < nt) bottom_adj_sweeps_cached<DIM, 2>(a, iterations, nt);
-        __syncthreads();
-        return;
-    }
-    if ((n + (int)blockDim.x - 1) / (int)blockDim.x <= 4) {
-        bottom_adj_sweeps_cached<DIM, 4>(a, iterations, blockDim.x);
-        __syncthreads();
-        return;
-    }
-    bottom_adj_half<DIM>(a, 1, false, true);
-    int colour = 1;
-    for (int k = 1; k < 2 * iterations; ++k) {
-        colour ^= 1;
-        bottom_adj_half<DIM>(a, colour, true, true);
-    }
-    bottom_adj_half<DIM>(a, colour ^ 1, true, false);
-}
-
-template <int DIM>
-__global__ void __launch_bounds__(1024) k_adj_bottom(AdjBottomArgs b) {
-    extern __shared__ float sm[];
-    float* sp = sm;
-    float* sb = sm + b.total;
-    float* sT = sm + 2 * b.total;
-    const int n0 = b.n[0][0] * b.n[0][1] * b.n[0][2];
-    for (int c = threadIdx.x; c < b.total; c += blockDim.x) {
-        sp[c] = c < n0 ? b.pbar0[c] : 0.f;
-        sb[c] = 0.f;
-        sT[c] = 0.f;
-    }
-    __syncthreads();
-    const int last = b.nlev - 1;
-    // down: post-smoothing^T, then prolongation^T into the (fresh) coarse pbar
-    for (int l = 0; l < last; ++l) {
-        const AdjLevel a = bottom_adj_level(b, l, sp, sb, sT);
-        bottom_adj_sweeps<DIM>(a, b.n_post);
-        const int cx = b.n[l + 1][0], cy = b.n[l + 1][1], cz = b.n[l + 1][2];
-        float* pc = sp + b.off[l + 1];
-        for (int q = threadIdx.x; q < cx * cy * cz; q += blockDim.x) {
-            const int X = q % cx, t = q / cx, Y = t % cy, Z = t / cy;
-            // per-axis coefficients of the fine window [2K-2, 2K+3] (0 outside the grid)
-            float wx[6], wy[6], wz[6];
-#pragma unroll
-            for (int j = 0; j < 6; ++j) {
-                const int x = 2 * X - 2 + j, y = 2 * Y - 2 + j, z = 2 * Z - 2 + j;
-                wx[j] = (x >= 0 && x < a.nx) ? prolong_coef(x, a.nx, cx, X) : 0.f;
-                wy[j] = (y >= 0 && y < a.ny) ? prolong_coef(y, a.ny, cy, Y) : 0.f;
-                wz[j] = DIM == 3 ? ((z >= 0 && z < a.nz) ? prolong_coef(z, a.nz, cz, Z) : 0.f) : (j == 2 ? 1.f : 0.f);
-            }
-            float s = 0.f;
-#pragma unroll
-            for (int k = 0; k < 6; ++k) {
-                if (wz[k] == 0.f) continue;
-                const int z = DIM == 3 ? 2 * Z - 2 + k : 0;
-#pragma unroll
-                for (int j = 0; j < 6; ++j) {
-                    if (wy[j] == 0.f) continue;
-                    const int y = 2 * Y - 2 + j;
-#pragma unroll
-                    for (int i = 0; i < 6; ++i)
-                        if (wx[i] != 0.f) s += wx[i] * wy[j] * wz[k] * a.pbar[idx3(2 * X - 2 + i, y, z, a.nx, a.ny)];
-                }
-            }
-            pc[q] = s;
-        }
-        __syncthreads();
-    }
-    if (b.cresp) {
-        // the coarsest sweeps as one product: bbar += D^T pbar, D = d(p after
-        // the sweeps)/d(right-hand side); the adjoint of their initial guess
-        // (zero) is not needed.  Threads split the sum over j into `parts`
-        // slices whose partial sums meet in the T arrays (unused outside the
-        // sweeps), then add in slice order.
-        const AdjLevel ac = bottom_adj_level(b, last, sp, sb, sT);
-        const int n = ac.nx * ac.ny * ac.nz;
-        int parts = (int)blockDim.x / n;
-        if (parts > b.total / n) parts = b.total / n;
-        if (parts < 1) parts = 1;
-        const int chunk = (n + parts - 1) / parts;
-        for (int t = threadIdx.x; t < n * parts; t += blockDim.x) {
-            const int i = t % n, part = t / n;
-            const int j0 = part * chunk, j1 = min(j0 + chunk, n);
-            const float* col = b.cresp + i;
-            float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
-            int j = j0;
-            for (; j + 4 <= j1; j += 4) {
-                s0 += __ldg(col + (size_t)j * n) * ac.pbar[j];
-                s1 += __ldg(col + (size_t)(j + 1) * n) * ac.pbar[j + 1];
-                s2 += __ldg(col + (size_t)(j + 2) * n) * ac.pbar[j + 2];
-                s3 += __ldg(col + (size_t)(j + 3) * n) * ac.pbar[j + 3];
-            }
-            for (; j < j1; ++j) s0 += __ldg(col + (size_t)j * n) * ac.pbar[j];
-            sT[t] = (s0 + s1) + (s2 + s3);
-        }
-        __syncthreads();
-        for (int i = threadIdx.x; i < n; i += blockDim.x) {
-            float acc = 0.f;
-            for (int part = 0; part < parts; ++part) acc += sT[part * n + i];
-            ac.bbar[i] += acc;
-        }
-        __syncthreads();
-    } else {
-        bottom_adj_sweeps<DIM>(bottom_adj_level(b, last, sp, sb, sT), b.n_coarse);
-    }
-    // up: residual + restriction^T, then pre-smoothing^T
-    for (int l = last - 1; l >= 0; --l) {
-        const AdjLevel a = bottom_adj_level(b, l, sp, sb, sT);
-        const int cx = b.n[l + 1][0], cy = b.n[l + 1][1], cz = b.n[l + 1][2];
-        const float* rcb = sb + b.off[l + 1];
-        const int n = a.nx * a.ny * a.nz;
-        for (int q = threadIdx.x; q < n; q += blockDim.x) {
-            const int x = q % a.nx, t = q / a.nx, y = t % a.ny, z = t / a.ny;
-            float wself, d;
-            bool fluid;
-            cell_weights<DIM, false>(a, x, y, z, wself, d, fluid);
-            const float rs = res_bar<DIM, false>(a, rcb, cx, cy, cz, x, y, z);
-            float nb = 0.f;
-            if (y + 1 < a.ny) nb += res_bar<DIM, false>(a, rcb, cx, cy, cz, x, y + 1, z);
-            if (y > 0) nb += res_bar<DIM, false>(a, rcb, cx, cy, cz, x, y - 1, z);
-            if (x + 1 < a.nx) nb += res_bar<DIM, false>(a, rcb, cx, cy, cz, x + 1, y, z);
-            if (x > 0) nb += res_bar<DIM, false>(a, rcb, cx, cy, cz, x - 1, y, z);
-            if constexpr (DIM == 3) {
-                if (z + 1 < a.nz) nb += res_bar<DIM, false>(a, rcb, cx, cy, cz, x, y, z + 1);
-                if (z > 0) nb += res_bar<DIM, false>(a, rcb, cx, cy, cz, x, y, z - 1);
-            }
-            a.pbar[q] += (d * rs - wself * nb) / a.hh;
-            a.bbar[q] += rs;
-        }
-        __syncthreads();
-        bottom_adj_sweeps<DIM>(a, b.n_pre);
-    }
-    for (int c = threadIdx.x; c < n0; c += blockDim.x) {
-        b.pbar0[c] = sp[c];
-        b.bbar0[c] += sb[c];
-    }
-}
-
-int bottom_start(const ss_sim* s) {
-    // finest level >= 1 from which the rest of the pyramid fits the block's shared memory
-    long long cum = 0;
-    int start = s->levels;
-    for (int l = s->levels - 1; l >= 1; --l) {
-        const long long n = (long long)s->lv[l].n[0] * s->lv[l].n[1] * s->lv[l].n[2];
-        if ((cum + n) * 12 > kBottomSmemBytes) break;
-        cum += n;
-        start = l;
-    }
-    return start;
-}
-
-static int adj_bottom(ss_sim* s, const ss_mg_schedule& mg, int L, const AdjScratch& w, cudaStream_t st) {
-    AdjBottomArgs b{};
-    b.nlev = s->levels - L;
-    int off = 0;
-    for (int l = 0; l < b.nlev; ++l) {
-        const ss::Level& lv = s->lv[L + l];
-        b.n[l][0] = lv.n[0]; b.n[l][1] = lv.n[1]; b.n[l][2] = lv.n[2];
-        b.off[l] = off;
-        b.hh[l] = lv.hh;
-        b.alpha[l] = s->alpha[L + l];
-        off += lv.n[0] * lv.n[1] * lv.n[2];
-    }
-    b.total = off;
-    b.pbar0 = w.pbar[L];
-    b.bbar0 = w.bbar[L];
-    b.n_pre = mg.n_pre; b.n_post = mg.n_post; b.n_coarse = mg.n_coarse;
-    b.oobA = s->enclosed ? 1.f : 0.f;
-    b.cresp = w.cresp;
-    const size_t smem = (size_t)3 * off * sizeof(float);
-    if (smem > (size_t)kBottomSmemBytes) return set_error(SS_E_INVALID, "adjoint bottom levels exceed shared memory");
-    cudaError_t e = s->dim == 3
-        ? cudaFuncSetAttribute(k_adj_bottom<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBottomSmemBytes)
-        : cudaFuncSetAttribute(k_adj_bottom<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBottomSmemBytes);
-    if (e != cudaSuccess) return check_cuda(e, "cudaFuncSetAttribute(k_adj_bottom)");
-    if (s->dim == 3) k_adj_bottom<3><<<1, 1024, smem, st>>>(b);
-    else k_adj_bottom<2><<<1, 1024, smem, st>>>(b);
-    s->nlaunch += 1;
-    return check_cuda(cudaGetLastError(), "k_adj_bottom");
-}
-
 // Transposed V-cycle from level L: on entry w.pbar[L] holds the adjoint of the
 // level's output pressure; on return it holds the adjoint of its input
 // pressure and w.bbar[L] has the right-hand side's adjoint added.
 static int adj_v_cycle_rec(ss_sim* s, const StepConsts& c, const ss_mg_schedule& mg, int L, const AdjScratch& w,
                            cudaStream_t st) {
     const AdjLevel a = adj_level(s, c, L, w);
-    if (L >= 1 && L >= s->bottom) return adj_bottom(s, mg, L, w, st);
+    if (L >= 1 && L >= s->coarse_from) return launch_adj_coarse(s, mg, L, w, st);
     if (L == s->levels - 1) return adj_sweeps(s, a, L, mg.n_coarse, st);
     TRY_ADJ(adj_sweeps(s, a, L, mg.n_post, st));
     const int cx = s->lv[L + 1].n[0], cy = s->lv[L + 1].n[1], cz = s->lv[L + 1].n[2];
@@ -1603,7 +1294,7 @@ static int adj_v_cycle_rec(ss_sim* s, const StepConsts& c, const ss_mg_schedule&
         k_adj_prolong<2, 6><<<gc, kB, 0, st>>>(a.pbar, a.nx, a.ny, a.nz, w.pbar[L + 1], cx, cy, cz);
     }
     s->nlaunch += 1;
-    TRY_ADJ(check_cuda(cudaMemsetAsync(w.bbar[L + 1], 0, nc * sizeof(float), st), "memset"));
+    if (L + 1 < s->coarse_from) TRY_ADJ(check_cuda(cudaMemsetAsync(w.bbar[L + 1], 0, nc * sizeof(float), st), "memset"));
     TRY_ADJ(adj_v_cycle_rec(s, c, mg, L + 1, w, st));
     // r_{L+1} = R(b_L - A p_L)
     dim3 gf = grid_of(a.nx, a.ny, a.nz, kB);

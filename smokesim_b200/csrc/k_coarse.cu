@@ -488,17 +488,11 @@ SS_D void visit(const CoarseArgs<T>& b, int l, bool up, cg::cluster_group* cl, i
     restrict_share<DIM, R>(cl, g, b.fine, b.lv[l + 1].n, b.r[l + 1], rank, ctas);
 }
 
-template <int DIM, typename T, typename R>
-__global__ void __launch_bounds__(kThreads) k_coarse(const __grid_constant__ CoarseArgs<T> b) {
-    cg::cluster_group cl = cg::this_cluster();
-    const int ctas = (int)cl.num_blocks(), rank = (int)cl.block_rank();
-    float* F = smf();
-    // pressures and ghost planes start at 0 (the initial guess, and the pressure
-    // outside the grid); every CTA has done so before a neighbour stores here
-    for (int i = threadIdx.x; i < b.nw; i += kThreads) F[i] = 0.f;
-    // the axes' prolongation taps depend on the sizes alone
+// the axes' prolongation taps, which depend on the sizes alone
+template <int DIM, typename T>
+SS_D void build_taps(const CoarseArgs<T>& b) {
     for (int l = 0; l + 1 < b.nlev; ++l) {
-        AxisTap* tap = reinterpret_cast<AxisTap*>(F + b.taps) + b.lv[l].tap;
+        AxisTap* tap = reinterpret_cast<AxisTap*>(smf() + b.taps) + b.lv[l].tap;
         const int nx = b.lv[l].n[0], ny = b.lv[l].n[1], nz = b.lv[l].n[2];
         for (int i = threadIdx.x; i < nx + ny + (DIM == 3 ? nz : 0); i += kThreads) {
             const int d = i < nx ? 0 : i < nx + ny ? 1 : 2, at = i - (d > 0 ? nx : 0) - (d > 1 ? ny : 0);
@@ -512,6 +506,17 @@ __global__ void __launch_bounds__(kThreads) k_coarse(const __grid_constant__ Coa
             tap[i] = v;
         }
     }
+}
+
+template <int DIM, typename T, typename R>
+__global__ void __launch_bounds__(kThreads) k_coarse(const __grid_constant__ CoarseArgs<T> b) {
+    cg::cluster_group cl = cg::this_cluster();
+    const int ctas = (int)cl.num_blocks(), rank = (int)cl.block_rank();
+    float* F = smf();
+    // pressures and ghost planes start at 0 (the initial guess, and the pressure
+    // outside the grid); every CTA has done so before a neighbour stores here
+    for (int i = threadIdx.x; i < b.nw; i += kThreads) F[i] = 0.f;
+    build_taps<DIM>(b);
     cl.sync();
     pdl_entry();
     // The level-0 sweeps since the last V-cycle have pushed the lower levels'
@@ -562,6 +567,196 @@ __global__ void __launch_bounds__(kThreads) k_coarse(const __grid_constant__ Coa
         if (l > 0) between(l, l - 1);
     }
     cl.sync();   // no CTA leaves while its shared memory may be read or written
+}
+
+// ------------------------------------------------------------- the transpose
+// The lower V-cycle's transpose (levels Lb..coarsest and back) over the same
+// slabs.  p is the adjoint of the levels' pressures, r that of their right-hand
+// sides (both natural, global); a thread keeps its cells' values of both in
+// registers through a visit's sweeps, and shared memory holds T, the quotient
+// each transposed update passes to its neighbours (k_adj_smooth in
+// k_adjoint.cu has the operator).  One visit is bound by its cluster barriers
+// and L2 round trips: 32^3, 16^3 and 8^3 with the response matrix take 54 us,
+// against 66 for the last two in one block and 21 launches and copies for 32^3.
+template <int DIM, int K>
+SS_D void adj_sweeps_slab(cg::cluster_group* cl, const Slab& g, const Cells<K>& c, const float (&ws)[2][K],
+                          float (&pb)[2][K], float (&bb)[2][K], int iterations, const Ghosts& gh) {
+    float* F = smf();
+    for (int it = 0; it < iterations; ++it) {
+#pragma unroll
+        for (int k = 1; k >= 0; --k) {
+            // the gather half of the colour before (none before the first), then this colour's transpose
+            float v[K];
+#pragma unroll
+            for (int j = 0; j < K; ++j)
+                v[j] = it == 0 && k == 1 ? pb[k][j] : pb[k][j] + ws[k][j] * cell_sum<DIM>(g, c, k, j);
+#pragma unroll
+            for (int j = 0; j < K; ++j) {
+                float t = div_recip(v[j], c.fs[k][j], c.yr[k][j]);
+                if (!recip_ok(v[j])) t = div_exact(v[j], c.fs[k][j]);
+                if (c.act[k][j]) {
+                    const int at = threadIdx.x + j * kThreads;
+                    F[(k ? g.w[1] : g.w[0]) + at] = t;
+                    gh.push(g, k, at, t);
+                    bb[k][j] -= g.hh * t;
+                }
+                pb[k][j] = c.act[k][j] ? 0.f : v[j];
+            }
+            if (cl) cl->sync();
+            else __syncthreads();
+        }
+    }
+    if (iterations > 0)
+#pragma unroll
+        for (int j = 0; j < K; ++j) pb[1][j] += ws[1][j] * cell_sum<DIM>(g, c, 1, j);
+}
+
+// One visit of level l: on the way down the post-smoothing's transpose (the
+// coarsest level's sweeps), on the way up that of residual, restriction and
+// pre-smoothing.
+template <int DIM, int K>
+SS_D void adj_visit(const CoarseArgs<float>& b, int l, bool up, cg::cluster_group* cl, int rank) {
+    const Slab g = slab_of<DIM>(b, l, rank);
+    const bool last = l == b.nlev - 1;
+    Cells<K> c;
+    load_cells<DIM>(g, b.alpha[l], b.alpha[l], b.oob_smooth, b.oob_resid, c);   // c.r: the cell's own alpha
+    float ws[2][K], pb[2][K], bb[2][K];
+#pragma unroll
+    for (int j = 0; j < K; ++j)
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            ws[k][j] = c.in[k][j] ? 1.f - c.r[k][j] : 0.f;
+            pb[k][j] = c.in[k][j] ? __ldcg(b.p[l] + c.index(g, k, j)) : 0.f;
+            bb[k][j] = up && c.in[k][j] ? __ldcg(b.r[l] + c.index(g, k, j)) : 0.f;
+        }
+    if (up) {
+        const int cx = b.lv[l + 1].n[0], cy = DIM == 3 ? b.lv[l + 1].n[1] : 1, cm = b.lv[l + 1].n[DIM == 3 ? 2 : 1];
+        auto parent = [&](int x, int y, int m) -> float {   // the residual's adjoint at a fluid cell
+            const int X = x >> 1, Y = DIM == 3 ? y >> 1 : 0, M = m >> 1;
+            return X < cx && Y < cy && M < cm ? __ldcg(b.r[l + 1] + (M * cy + Y) * cx + X) * (DIM == 3 ? 0.125f : 0.25f) : 0.f;
+        };
+#pragma unroll
+        for (int j = 0; j < K; ++j)
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                if (!c.in[k][j]) continue;
+                const float* f = c.f[k][j];   // 0: solid or out of grid
+                const int x = c.x(k, j), y = c.y[j], m = c.m[j];
+                const float rs = c.live[k][j] ? parent(x, y, m) : 0.f;
+                float nb = 0.f;
+                if (f[0] > 0.f) nb += DIM == 3 ? parent(x, y + 1, m) : parent(x, y, m + 1);
+                if (f[1] > 0.f) nb += DIM == 3 ? parent(x, y - 1, m) : parent(x, y, m - 1);
+                if (f[2] > 0.f) nb += parent(x + 1, y, m);
+                if (f[3] > 0.f) nb += parent(x - 1, y, m);
+                if constexpr (DIM == 3) {
+                    if (f[4] > 0.f) nb += parent(x, y, m + 1);
+                    if (f[5] > 0.f) nb += parent(x, y, m - 1);
+                }
+                pb[k][j] += (c.fr[k][j] * rs - ws[k][j] * nb) / g.hh;
+                bb[k][j] += rs;
+            }
+    }
+    // the gather takes its neighbours' T unweighted; a solid neighbour's is 0
+#pragma unroll
+    for (int j = 0; j < K; ++j)
+#pragma unroll
+        for (int k = 0; k < 2; ++k)
+#pragma unroll
+            for (int d = 0; d < 6; ++d) c.f[k][j][d] = c.f[k][j][d] > 0.f ? 1.f : 0.f;
+    const Ghosts gh(cl, g, rank);
+    adj_sweeps_slab<DIM>(cl, g, c, ws, pb, bb, up ? b.n_pre : last ? b.n_coarse : b.n_post, gh);
+#pragma unroll
+    for (int j = 0; j < K; ++j)
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            if (!c.in[k][j]) continue;
+            if (!up) b.p[l][c.index(g, k, j)] = pb[k][j];
+            b.r[l][c.index(g, k, j)] = bb[k][j];
+        }
+}
+
+// Transpose of the prolongation onto level l (k_adj_prolong's sums), by all
+// threads of the cluster: the fine window of coarse index K is [2K-2, 2K+3].
+template <int DIM>
+SS_D void adj_prolong_share(const CoarseArgs<float>& b, int l, int first, int threads) {
+    const int* cn = b.lv[l].n;
+    const int* fn = b.lv[l - 1].n;
+    const AxisTap* tap = reinterpret_cast<const AxisTap*>(smf() + b.taps) + b.lv[l - 1].tap;
+    const int n = cn[0] * cn[1] * (DIM == 3 ? cn[2] : 1);
+    for (int i = first; i < n; i += threads) {
+        const int X = i % cn[0], t = i / cn[0], Y = t % cn[1], Z = t / cn[1];
+        auto coef = [&](int d, int x, int K) -> float {
+            if (x < 0 || x >= fn[d]) return 0.f;
+            const AxisTap v = tap[x + (d > 0 ? fn[0] : 0) + (d > 1 ? fn[1] : 0)];
+            return (v.lo == K ? 1.f - v.w : 0.f) + (v.hi == K ? v.w : 0.f);
+        };
+        float wx[6], wy[6];
+#pragma unroll
+        for (int q = 0; q < 6; ++q) {
+            wx[q] = coef(0, 2 * X - 2 + q, X);
+            wy[q] = coef(1, 2 * Y - 2 + q, Y);
+        }
+        float s = 0.f;
+        for (int k = 0; k < (DIM == 3 ? 6 : 1); ++k) {
+            const int z = DIM == 3 ? 2 * Z - 2 + k : 0;
+            const float wz = DIM == 3 ? coef(2, z, Z) : 1.f;
+            if (wz == 0.f) continue;
+            float v[6][6];
+#pragma unroll
+            for (int j = 0; j < 6; ++j)
+#pragma unroll
+                for (int q = 0; q < 6; ++q)
+                    v[j][q] = wy[j] != 0.f && wx[q] != 0.f
+                                  ? __ldcg(b.p[l - 1] + (z * fn[1] + 2 * Y - 2 + j) * fn[0] + 2 * X - 2 + q) : 0.f;
+#pragma unroll
+            for (int j = 0; j < 6; ++j) {
+                float row = 0.f;
+#pragma unroll
+                for (int q = 0; q < 6; ++q) row += wx[q] * v[j][q];
+                s += wz * wy[j] * row;
+            }
+        }
+        b.p[l][i] = s;
+    }
+}
+
+template <int DIM>
+__global__ void __launch_bounds__(kThreads) k_adj_coarse(const __grid_constant__ CoarseArgs<float> b) {
+    cg::cluster_group cl = cg::this_cluster();
+    const int ctas = (int)cl.num_blocks(), rank = (int)cl.block_rank();
+    const int first = rank * kThreads + (int)threadIdx.x, threads = ctas * kThreads;
+    float* F = smf();
+    for (int i = threadIdx.x; i < b.nw; i += kThreads) F[i] = 0.f;   // T outside the grid and of solid cells
+    build_taps<DIM>(b);
+    cl.sync();
+    auto run = [&](int l, bool up) {
+        const CoarseLevel& v = b.lv[l];
+        if (!v.solo || rank == 0) {
+            const int ncol = (v.n[0] + 1) / 2 * (DIM == 3 ? v.n[1] : 1);
+            if (v.planes * ncol > kThreads) adj_visit<DIM, 2>(b, l, up, v.solo ? nullptr : &cl, rank);
+            else adj_visit<DIM, 1>(b, l, up, v.solo ? nullptr : &cl, rank);
+        }
+        cl.sync();
+    };
+    const int last = b.nlev - 1;
+    for (int l = 0; l < last; ++l) {
+        run(l, false);
+        adj_prolong_share<DIM>(b, l + 1, first, threads);
+        cl.sync();
+    }
+    if (b.cmat) {
+        // the coarsest sweeps as one product: r = D^T p, D[j n + i] = dp_j / dr_i
+        const int n = b.lv[last].n[0] * b.lv[last].n[1] * b.lv[last].n[2];
+        for (int i = threadIdx.x; i < n; i += kThreads) F[b.fine + i] = __ldcg(b.p[last] + i);
+        __syncthreads();
+        coarse_matrix_partials<false>(b.cmat, F + b.fine, b.cpart, n, first, threads);
+        cl.sync();
+        coarse_matrix_fold<true, float>(b.cpart, b.r[last], n, first, threads);
+        cl.sync();
+    } else {
+        run(last, false);
+    }
+    for (int l = last - 1; l >= 0; --l) run(l, true);
 }
 
 // ------------------------------------------------------------------ host
@@ -639,28 +834,38 @@ static void coarse_config(int ctas, size_t smem, cudaLaunchConfig_t* cfg, cudaLa
     cfg->numAttrs = 1;
 }
 
-template <int DIM, typename T>
-static cudaError_t coarse_attributes() {
-    const cudaError_t e = cudaFuncSetAttribute(k_coarse<DIM, T, T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+template <typename K>
+static cudaError_t coarse_attributes(K* kernel) {
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e != cudaSuccess) cudaGetLastError();   // clusters of at most 8 then
-    return cudaFuncSetAttribute(k_coarse<DIM, T, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCoarseSmem);
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCoarseSmem);
 }
 
-template <int DIM, typename T>
-static bool cluster_placeable(int ctas) {
+template <typename K>
+static bool cluster_placeable(K* kernel, int ctas) {
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute at[1];
     int active = 0;
     coarse_config(ctas, kCoarseSmem, &cfg, at);
-    const cudaError_t e = cudaOccupancyMaxActiveClusters(&active, k_coarse<DIM, T, T>, &cfg);
+    const cudaError_t e = cudaOccupancyMaxActiveClusters(&active, kernel, &cfg);
     if (e != cudaSuccess) cudaGetLastError();   // an unsupported size is not an error of the solve
     return e == cudaSuccess && active >= 1;
 }
 
 template <int DIM>
+static cudaError_t coarse_attributes_all() {
+    cudaError_t e = coarse_attributes(k_coarse<DIM, float, float>);
+    if (e == cudaSuccess) e = coarse_attributes(k_coarse<DIM, __half, __half>);
+    if (e == cudaSuccess) e = coarse_attributes(k_coarse<DIM, __nv_bfloat16, __nv_bfloat16>);
+    if (e == cudaSuccess) e = coarse_attributes(k_adj_coarse<DIM>);
+    return e;
+}
+
+template <int DIM>
 static int largest_cluster() {
     for (int c = kMaxCtas; c > 1; c /= 2)
-        if (cluster_placeable<DIM, float>(c) && cluster_placeable<DIM, __half>(c) && cluster_placeable<DIM, __nv_bfloat16>(c))
+        if (cluster_placeable(k_coarse<DIM, float, float>, c) && cluster_placeable(k_coarse<DIM, __half, __half>, c) &&
+            cluster_placeable(k_coarse<DIM, __nv_bfloat16, __nv_bfloat16>, c) && cluster_placeable(k_adj_coarse<DIM>, c))
             return c;
     return 1;
 }
@@ -678,10 +883,7 @@ int coarse_setup(ss_sim* s) {
         std::lock_guard<std::mutex> lock(mu);
         int& c = known[4 * dev + s->dim];
         if (!c) {
-            cudaError_t e = s->dim == 3 ? coarse_attributes<3, float>() : coarse_attributes<2, float>();
-            if (e == cudaSuccess) e = s->dim == 3 ? coarse_attributes<3, __half>() : coarse_attributes<2, __half>();
-            if (e == cudaSuccess)
-                e = s->dim == 3 ? coarse_attributes<3, __nv_bfloat16>() : coarse_attributes<2, __nv_bfloat16>();
+            const cudaError_t e = s->dim == 3 ? coarse_attributes_all<3>() : coarse_attributes_all<2>();
             if (e != cudaSuccess) return check_cuda(e, "coarse cluster attributes");
             c = s->dim == 3 ? largest_cluster<3>() : largest_cluster<2>();
         }
@@ -692,14 +894,16 @@ int coarse_setup(ss_sim* s) {
     return SS_OK;
 }
 
+// The arguments both kernels share; returns the cluster's CTAs (0: none fits) and
+// its shared memory in floats.
 template <int DIM, typename T>
-static int launch_coarse_t(ss_sim* s, const ss_mg_schedule& mg, int L, T* const* p, T* const* r, bool p_zero, cudaStream_t st) {
+static int coarse_args(const ss_sim* s, const ss_mg_schedule& mg, int L, T* const* p, T* const* r, CoarseArgs<T>& b,
+                       long long* floats) {
     const int ctas = coarse_ctas(s, L, s->coarse_max_ctas);
-    if (!ctas) return set_error(SS_E_INVALID, "level too large for the coarse cluster");
-    CoarseArgs<T> b{};
+    if (!ctas) return 0;
     b.nlev = s->levels - L;
     long long nw = 0, taps = 0;
-    const long long floats = coarse_floats(s, L, ctas, &nw, &taps);
+    *floats = coarse_floats(s, L, ctas, &nw, &taps);
     int w = 0, tap = 0;
     for (int l = 0; l < b.nlev; ++l) {
         const ss::Level& lv = s->lv[L + l];
@@ -718,6 +922,15 @@ static int launch_coarse_t(ss_sim* s, const ss_mg_schedule& mg, int L, T* const*
     b.nw = b.taps = (int)nw;
     b.fine = (int)(nw + 2 * taps);
     b.n_pre = mg.n_pre; b.n_post = mg.n_post; b.n_coarse = mg.n_coarse;
+    return ctas;
+}
+
+template <int DIM, typename T>
+static int launch_coarse_t(ss_sim* s, const ss_mg_schedule& mg, int L, T* const* p, T* const* r, bool p_zero, cudaStream_t st) {
+    CoarseArgs<T> b{};
+    long long floats = 0;
+    const int ctas = coarse_args<DIM>(s, mg, L, p, r, b, &floats);
+    if (!ctas) return set_error(SS_E_INVALID, "level too large for the coarse cluster");
     b.quirks = mg.ref_quirks ? 1 : 0;
     b.p_zero = p_zero ? 1 : 0;
     b.oob_smooth = smooth_oob(s, mg.ref_quirks);
@@ -749,6 +962,31 @@ int launch_coarse_mixed(ss_sim* s, const ss_mg_schedule& mg, int L, int prec, cu
     if (prec == SS_PREC_MIXED)
         return launch_coarse_d<__half>(s, mg, L, (__half* const*)s->cp, (__half* const*)s->cr, true, st);
     return launch_coarse_d<__nv_bfloat16>(s, mg, L, (__nv_bfloat16* const*)s->cp, (__nv_bfloat16* const*)s->cr, true, st);
+}
+
+// pbar, bbar: adjoint pressures and right-hand sides of all levels; the former's of
+// level L is read, the latter's written.  cresp: the coarsest sweeps' response
+// matrix (layout 0), or null; cpart: kProductLanes floats with it.
+template <int DIM>
+static int launch_adj_coarse_t(ss_sim* s, const ss_mg_schedule& mg, int L, const AdjScratch& w, cudaStream_t st) {
+    CoarseArgs<float> b{};
+    long long floats = 0;
+    const int ctas = coarse_args<DIM>(s, mg, L, w.pbar, w.bbar, b, &floats);
+    if (!ctas) return set_error(SS_E_INVALID, "level too large for the coarse cluster");
+    b.oob_smooth = b.oob_resid = s->enclosed ? 1.f : 0.f;
+    b.cmat = w.cresp;
+    b.cpart = w.cpart;
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute at[1];
+    coarse_config(ctas, (size_t)floats * sizeof(float), &cfg, at);
+    cfg.stream = st;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, k_adj_coarse<DIM>, b);
+    s->nlaunch += 1;
+    return check_cuda(e, "k_adj_coarse");
+}
+
+int launch_adj_coarse(ss_sim* s, const ss_mg_schedule& mg, int L, const AdjScratch& w, cudaStream_t st) {
+    return s->dim == 3 ? launch_adj_coarse_t<3>(s, mg, L, w, st) : launch_adj_coarse_t<2>(s, mg, L, w, st);
 }
 
 // Response of the coarsest level's smoothing to unit right-hand sides: block

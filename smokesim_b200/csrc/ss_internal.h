@@ -98,7 +98,6 @@ struct ss_sim {
     int svel_active = 0;
 
     int levels = 0;
-    int bottom = 0;            // first level of the adjoint's single-block lower V-cycle (== levels: none)
     ss::Level lv[SS_MAX_LEVELS];
     float* p[SS_MAX_LEVELS] = {};
     float* r[SS_MAX_LEVELS] = {};
@@ -219,9 +218,6 @@ int launch_solid_pyramid(ss_sim* s, cudaStream_t st);
 int coarse_setup(ss_sim* s);
 int launch_coarse(ss_sim* s, const ss_mg_schedule& mg, int L, cudaStream_t st, bool p_zero = false);
 int launch_coarse_mixed(ss_sim* s, const ss_mg_schedule& mg, int L, int prec, cudaStream_t st);
-// the adjoint's single-block lower V-cycle
-constexpr int kBottomSmemBytes = 160 * 1024;
-int bottom_start(const ss_sim* s);
 // level 0 on colour-split arrays during a solve (k_rb.cu)
 bool rb_supported(const ss_sim* s, int quirks);
 int launch_rb_convert(ss_sim* s, bool split, cudaStream_t st);
@@ -289,15 +285,16 @@ struct AdjScratch {
     float* bbar[SS_MAX_LEVELS];
     float* T[SS_MAX_LEVELS];
     // response matrix of the coarsest level's sweeps (launch_coarse_response);
-    // null: the bottom solve's adjoint transposes the sweeps one by one
+    // null: the lower V-cycle's transpose takes the sweeps one by one
     const float* cresp;
+    float* cpart;   // with it: kProductLanes floats
 };
 // coarsest levels up to this many cells get a response matrix (4 MiB)
 constexpr int kCoarseResponseMax = 1024;
-// lanes of the coarsest level's matrix product (k_mg.cu, coarse_parts): one
-// 16-block cluster of 1024 threads
+// items of the coarsest level's matrix product (coarse_level.cuh, coarse_parts)
 constexpr int kProductLanes = 16384;
 int launch_coarse_response(ss_sim* s, int iters, float* D, cudaStream_t st);
+int launch_adj_coarse(ss_sim* s, const ss_mg_schedule& mg, int L, const AdjScratch& w, cudaStream_t st);
 int update_coarse_matrix(ss_sim* s, const ss_mg_schedule& mg, cudaStream_t st);
 // Scratch of the deterministic (owner-computes) adjoint scatters; a null
 // AdjOwner selects the atomic scatter-adds.
