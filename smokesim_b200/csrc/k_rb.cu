@@ -216,8 +216,8 @@ struct RbPlane {
 // takes the same three operations for every f: q0 = a y, r = a - f q0, q0 + r y
 // with y = RN(1/f) - div_by_count's steps, which for f = 6 halve everything by
 // an exact factor - with {f, y} from a table indexed by the mask byte.  Tiny
-// dividends, where those steps are not exact, are redone by div_by_count out of
-// line.  Threads fill warps across rows, so that short rows leave no lane idle.
+// dividends, where those steps are not exact, and -0, whose sign they lose, are
+// redone by div_by_count out of line.  Threads fill warps across rows, so that short rows leave no lane idle.
 // A half-sweep in a replayed solve: 5.9 us at 128^3 (8.8 with a selected
 // reciprocal and a row of threads per grid row), 8.1 at 192x128x160 (10.4), 3.5 at
 // 64^3 (4.5; a launch's latency), 23 at 256^3 (23.5; 4.8 TB/s of the 6.5 a copy
@@ -315,7 +315,7 @@ __global__ void __launch_bounds__(256) k_rb_smooth4(float* __restrict__ pc, cons
                 }
             }
             a[k] = sum - f4(cur.rhs, k);
-            tiny = tiny || (fabsf(a[k]) < 7.52316385e-37f && a[k] != 0.f);
+            tiny = tiny || (fabsf(a[k]) < 7.52316385e-37f && __float_as_uint(a[k]) != 0u);
         }
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
