@@ -779,74 +779,74 @@ constexpr int kUpdPlanes = 8;
 
 // p0_out (FP64 pressure only): also store each cell's pressure rounded to
 // FP32 - the pressure field of the API - in the same pass.
+// One thread per cell column takes the cells' low faces, and the faces past the
+// last cell of a row or column beside them: a grid of nx x ny threads, where one of
+// (nx + 1) x (ny + 1) leaves a ninth of the warps of a 256-cell row nearly empty.
+// Bound by memory latency, six blocks an SM: 124 us at 256^3 with the FP64 pressure
+// (178 with a face position a thread, a bounds test and a neighbour's flags per
+// face; 127 at five blocks), 17.4 at 128^3 in FP32 (25.5), 4.1 at 64^3 (5.4).
 template <int DIM, typename P = float>
-__global__ void __launch_bounds__(256) k_update_velocity(FluidArgs a, const P* __restrict__ p, int planes,
+__global__ void __launch_bounds__(256, 6) k_update_velocity(FluidArgs a, const P* __restrict__ p, int planes,
                                                          double k64 = 0.0, float* __restrict__ p0_out = nullptr) {
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     const int y = blockIdx.y * blockDim.y + threadIdx.y;
     const int nx = a.nx, ny = a.ny, nz = a.nz;
+    if (x >= nx || y >= ny) return;
     const int zb = blockIdx.z * planes;
     const int zend = min(zb + planes, DIM == 3 ? nz + 1 : 1);
-    const bool inxy = x < nx && y < ny;
+    const int pl = nx * ny;
     P p_back = P(0);
     bool s_back = false;
-    if (DIM == 3 && inxy && zb > 0) {
+    if (DIM == 3 && zb > 0) {
         p_back = __ldg(p + idx3(x, y, zb - 1, nx, ny));
         s_back = a.flags[idx3(x, y, zb - 1, nx, ny)] & F_SOLID;
     }
-    // a plane's loads, issued one plane ahead so they are in flight across
-    // the plane before: the cell's pressure and solid flag, and per x / y face
-    // the face velocity and the lower cell's pressure and flag (z faces take
-    // the lower cell from the previous plane); every address is in range
+    // a plane's loads, issued one plane ahead so they are in flight across the
+    // plane before: the cell's pressure and flags and, per face, its velocity and
+    // (x, y) the lower cell's pressure; z faces take the lower cell from the
+    // previous plane.  A pressure outside the grid is 0.
     struct Plane {
         P pc, plo[2];
         float src[3];
-        bool sc, slo[2];
+        uint8_t fl;
     };
     auto fetch = [&](int z, Plane& L) {
-        const bool in = inxy && z < nz;
-        L.pc = in ? __ldg(p + idx3(x, y, z, nx, ny)) : P(0);
-        L.sc = in && (a.flags[idx3(x, y, z, nx, ny)] & F_SOLID);
-#pragma unroll
-        for (int comp = 0; comp < DIM; ++comp) {
-            const int ax = nx + (comp == 0), ay = ny + (comp == 1), az = nz + (comp == 2);
-            L.src[comp] = 0.f;
-            if (comp < 2) { L.plo[comp] = P(0); L.slo[comp] = false; }
-            if (x >= ax || y >= ay || z >= az) continue;
-            const float* __restrict__ src = comp == 0 ? a.u : comp == 1 ? a.v : a.w;
-            L.src[comp] = __ldg(src + idx3(x, y, z, ax, ay));
-            if (comp < 2) {
-                const int xm = x - (comp == 0), ym = y - (comp == 1);
-                L.slo[comp] = solid_oob0(a.flags, xm, ym, z, nx, ny, nz);
-                L.plo[comp] = (xm < 0 || ym < 0) ? P(0) : __ldg(p + idx3(xm, ym, z, nx, ny));
-            }
-        }
+        const int c = z * pl + y * nx + x;
+        if constexpr (DIM == 3) L.src[2] = __ldg(a.w + c);
+        L.pc = L.plo[0] = L.plo[1] = P(0);
+        L.src[0] = L.src[1] = 0.f;
+        L.fl = 0;
+        if (z >= nz) return;
+        L.pc = __ldg(p + c);
+        L.fl = a.flags[c];
+        L.src[0] = __ldg(a.u + z * (nx + 1) * ny + y * (nx + 1) + x);
+        L.src[1] = __ldg(a.v + z * nx * (ny + 1) + y * nx + x);
+        if (x > 0) L.plo[0] = __ldg(p + c - 1);
+        if (y > 0) L.plo[1] = __ldg(p + c - nx);
+    };
+    auto moved = [&](float src, P hi, P lo) -> float {
+        if constexpr (std::is_same<P, double>::value) return (float)((double)src + k64 * (hi - lo));
+        else return src + a.c.k_upd * (hi - lo);
     };
     Plane cur;
     fetch(zb, cur);
     for (int z = zb; z < zend; ++z) {
         Plane nxt = cur;
         if (z + 1 < zend) fetch(z + 1, nxt);
-        const bool in = inxy && z < nz;
+        const int c = z * pl + y * nx + x;
         const P pc = cur.pc;
-        const bool sc = cur.sc;
-        if (p0_out && in) p0_out[idx3(x, y, z, nx, ny)] = (float)pc;
-#pragma unroll
-        for (int comp = 0; comp < DIM; ++comp) {
-            const int ax = nx + (comp == 0), ay = ny + (comp == 1), az = nz + (comp == 2);
-            if (x >= ax || y >= ay || z >= az) continue;
-            float* __restrict__ dst = comp == 0 ? a.uo : comp == 1 ? a.vo : a.wo;
-            const int i = idx3(x, y, z, ax, ay);
-            const bool s_lo = comp == 2 ? s_back : cur.slo[comp < 2 ? comp : 0];
-            if (sc || s_lo) {
-                const float* sv = comp == 0 ? a.sv0 : comp == 1 ? a.sv1 : a.sv2;
-                dst[i] = (in && sv) ? sv[idx3(x, y, z, nx, ny)] : 0.f;
-                continue;
-            }
-            const P plo = comp == 2 ? p_back : cur.plo[comp < 2 ? comp : 0];
-            if constexpr (std::is_same<P, double>::value) dst[i] = (float)((double)cur.src[comp] + k64 * (pc - plo));
-            else dst[i] = cur.src[comp] + a.c.k_upd * (pc - plo);
+        const bool sc = cur.fl & F_SOLID;
+        if (z < nz) {
+            if (p0_out) p0_out[c] = (float)pc;
+            const int iu = z * (nx + 1) * ny + y * (nx + 1) + x, iv = z * nx * (ny + 1) + y * nx + x;
+            const bool su = sc || (x > 0 && (cur.fl & F_LEFT)), sv = sc || (y > 0 && (cur.fl & F_BOTTOM));
+            a.uo[iu] = su ? (a.sv0 ? a.sv0[c] : 0.f) : moved(cur.src[0], pc, cur.plo[0]);
+            a.vo[iv] = sv ? (a.sv1 ? a.sv1[c] : 0.f) : moved(cur.src[1], pc, cur.plo[1]);
+            if (x == nx - 1) a.uo[iu + 1] = sc ? 0.f : moved(__ldg(a.u + iu + 1), P(0), pc);
+            if (y == ny - 1) a.vo[iv + nx] = sc ? 0.f : moved(__ldg(a.v + iv + nx), P(0), pc);
         }
+        if constexpr (DIM == 3)
+            a.wo[c] = sc || s_back ? (z < nz && a.sv2 ? a.sv2[c] : 0.f) : moved(cur.src[2], pc, p_back);
         p_back = pc;
         s_back = sc;
         cur = nxt;
@@ -856,8 +856,8 @@ __global__ void __launch_bounds__(256) k_update_velocity(FluidArgs a, const P* _
 int launch_update_velocities(ss_sim* s, const StepConsts& c, cudaStream_t st) {
     FluidArgs a = fluid_args(s, c);
     dim3 b(32, 8, 1);
-    const int planes = z_planes((long long)((s->nx + 32) / 32) * ((s->ny + 8) / 8), s->nz + 1, kUpdPlanes);
-    dim3 g = grid_for(s->nx + 1, s->ny + 1, s->dim == 3 ? (s->nz + planes) / planes : 1, b);
+    const int planes = z_planes((long long)((s->nx + 31) / 32) * ((s->ny + 7) / 8), s->nz + 1, kUpdPlanes);
+    dim3 g = grid_for(s->nx, s->ny, s->dim == 3 ? (s->nz + planes) / planes : 1, b);
     if (s->dim == 3) k_update_velocity<3><<<g, b, 0, st>>>(a, s->p[0], planes);
     else k_update_velocity<2><<<g, b, 0, st>>>(a, s->p[0], planes);
     for (int d = 0; d < s->dim; ++d) s->vi[d] ^= 1;
@@ -868,8 +868,8 @@ int launch_update_velocities(ss_sim* s, const StepConsts& c, cudaStream_t st) {
 int launch_update_velocities_p64(ss_sim* s, const StepConsts& c, cudaStream_t st, float* p0_out) {
     FluidArgs a = fluid_args(s, c);
     dim3 b(32, 8, 1);
-    const int planes = z_planes((long long)((s->nx + 32) / 32) * ((s->ny + 8) / 8), s->nz + 1, kUpdPlanes);
-    dim3 g = grid_for(s->nx + 1, s->ny + 1, s->dim == 3 ? (s->nz + planes) / planes : 1, b);
+    const int planes = z_planes((long long)((s->nx + 31) / 32) * ((s->ny + 7) / 8), s->nz + 1, kUpdPlanes);
+    dim3 g = grid_for(s->nx, s->ny, s->dim == 3 ? (s->nz + planes) / planes : 1, b);
     const double k64 = -(double)c.dt / ((double)c.rho * (double)s->h);
     if (s->dim == 3) k_update_velocity<3, double><<<g, b, 0, st>>>(a, s->p64, planes, k64, p0_out);
     else k_update_velocity<2, double><<<g, b, 0, st>>>(a, s->p64, planes, k64, p0_out);

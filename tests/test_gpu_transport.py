@@ -1,5 +1,5 @@
-"""Advection of velocities and smoke where one thread per cell takes the faces
-around it: grids thinner than a block, one cell past a block's edge, wind at the
+"""Advection of velocities and smoke and the projection update, where one thread per
+cell takes the faces around it: grids thinner than a block, one cell past a block's edge, wind at the
 low face of every axis, traces that end exactly on the last cell or far outside.
 Bit for bit against the FP32 oracle."""
 import numpy as np
@@ -22,7 +22,7 @@ THIN = [
 
 @pytest.mark.parametrize("name,dim,n,nch,enc", THIN)
 @pytest.mark.parametrize("mask", [abi.STAGE_ADVECT_VELOCITIES, abi.STAGE_ADVECT_VELOCITIES | abi.STAGE_APPLY_BUOYANCY,
-                                  abi.STAGE_ADVECT_SMOKE])
+                                  abi.STAGE_ADVECT_SMOKE, abi.STAGE_UPDATE_VELOCITIES])
 @pytest.mark.parametrize("vel", ["random", "integer", "far"])
 def test_transport_edges_bitwise(name, dim, n, nch, enc, mask, vel):
     g, o = make_pair(dim, n, nch, enc, seed=61, min_coarse=3, t_amb=0.5)
