@@ -36,9 +36,10 @@
 // of 24x18x15 cells 86 us (in one block 875 us: 0.5 against 5.4 us a half-sweep).
 //
 // The arithmetic per cell is that of smooth_cell / residual_cell (a neighbour
-// outside the grid has weight 0 in place of its 0 pressure; its weight still
-// counts in the divisor), the restriction's sum order and the prolongation's
-// expression are those of k_mg.cu: the same values as the per-level launches.
+// outside the grid is a 0 read from shared memory; its weight still counts in the
+// divisor), the restriction's sum order and the prolongation's expression are
+// those of k_mg.cu: the same values as the per-level launches, infinities and NaN
+// included.
 #include <algorithm>
 #include <cmath>
 #include <map>
@@ -57,6 +58,7 @@ namespace ss {
 constexpr int kThreads = 512;   // 128 registers a thread for two cells of each colour
 constexpr int kCells = 2;       // cells of each colour per thread, at most
 constexpr int kMaxCtas = 16;
+constexpr int kZeros = 32;      // floats of 0, one in each bank, in front of the pressures
 
 // div_recip may take this dividend
 SS_D bool recip_ok(float a) {
@@ -81,7 +83,7 @@ struct CoarseArgs {
     T* p[SS_MAX_LEVELS];
     T* r[SS_MAX_LEVELS];
     const float* alpha[SS_MAX_LEVELS];
-    int nw, taps, fine;   // floats of all pressures; offsets of the tap tables (entries follow) and of the residuals
+    int nw, taps, fine;   // floats of the zeros and all pressures; offsets of the tap tables (entries follow) and of the residuals
     int n_pre, n_post, n_coarse, quirks;
     int p_zero;           // the first level's pressure is 0: not read
     float oob_smooth, oob_resid;
@@ -150,6 +152,7 @@ struct Cells {
     float f[2][K][6], fs[2][K], yr[2][K], fr[2][K], r[2][K];
     int x2[K], y[K], m[K];   // the pair's even x, its row and plane
     int odd[K];              // x parity of the red cell (the black one's is the other)
+    int nb[2][K][6];         // the neighbours' places in shared memory (outside the grid: one of the zeros)
     bool act[2][K];          // updated by the sweeps
     bool live[2][K];         // not solid
     bool in[2][K];           // a cell of the grid
@@ -170,6 +173,26 @@ SS_D void load_cells(const Slab& g, const float* __restrict__ alpha, const T* r,
         e[4] = DIM == 3 && c.m[j] + 1 < g.nm;
         e[5] = DIM == 3 && c.m[j] > 0;
     };
+    // A neighbour outside the grid is read as 0, from the bank that its place in the
+    // packed order has: no test in the sweeps and no bank conflict.  In 3D
+    // formed after the loads are issued (reverse pass of a 64^3 solve of 8 V-cycles
+    // 1661 us, 1708 before them), in 2D before them (8 V-cycles at 256^2 with 16-bit
+    // storage 511 us; 559 after them, where those forms spill).
+    auto places = [&](int k, int j) {
+        bool e[6];
+        edges(k, j, e);
+        const int at = (k ? g.w[0] : g.w[1]) + threadIdx.x + j * kThreads, right = c.odd[j] ^ k, ts = DIM == 3 ? g.hx : g.ncol;
+        auto place = [&](int to, bool inside) { return (at + to) & (c.in[k][j] && inside ? -1 : kZeros - 1); };
+        int* nb = c.nb[k][j];
+        nb[0] = place(ts, e[0]);
+        nb[1] = place(-ts, e[1]);
+        nb[2] = place(right, e[2]);
+        nb[3] = place(right - 1, e[3]);
+        if constexpr (DIM == 3) {
+            nb[4] = place(g.ncol, e[4]);
+            nb[5] = place(-g.ncol, e[5]);
+        }
+    };
 #pragma unroll
     for (int j = 0; j < K; ++j) {
         const int q = threadIdx.x + j * kThreads, pl = q / g.ncol, col = q - pl * g.ncol, y = col / g.hx;
@@ -181,6 +204,7 @@ SS_D void load_cells(const Slab& g, const float* __restrict__ alpha, const T* r,
         for (int k = 0; k < 2; ++k) {
             c.in[k][j] = q < g.cnt && c.x(k, j) < g.nx;
             const int i = c.index(g, k, j), off[6] = {g.nx, -g.nx, 1, -1, g.nx * g.ny, -g.nx * g.ny};
+            if constexpr (DIM == 2) places(k, j);
             bool e[6];
             edges(k, j, e);
             a[k][j][6] = 1.f;
@@ -192,6 +216,11 @@ SS_D void load_cells(const Slab& g, const float* __restrict__ alpha, const T* r,
             for (int d = 0; d < 6; ++d) a[k][j][d] = c.in[k][j] && e[d] ? __ldg(alpha + i + off[d]) : 1.f;
         }
     }
+    if constexpr (DIM == 3)
+#pragma unroll
+        for (int j = 0; j < K; ++j)
+#pragma unroll
+            for (int k = 0; k < 2; ++k) places(k, j);
 #pragma unroll
     for (int j = 0; j < K; ++j)
 #pragma unroll
@@ -225,18 +254,16 @@ SS_D void load_cells(const Slab& g, const float* __restrict__ alpha, const T* r,
 
 // neighbour sum of cell j of colour k, in smooth_cell's order
 template <int DIM, int K>
-SS_D float cell_sum(const Slab& g, const Cells<K>& c, int k, int j) {
-    const float* P = smf() + (k ? g.w[0] : g.w[1]);
-    const int q = threadIdx.x + j * kThreads < g.cnt ? threadIdx.x + j * kThreads : 0;
-    const int ts = DIM == 3 ? g.hx : g.ncol;
+SS_D float cell_sum(const Cells<K>& c, int k, int j) {
+    const float* P = smf();
     const float* f = c.f[k][j];
-    float s = P[q + ts] * f[0] + P[q - ts] * f[1];
-    const int right = q + (c.odd[j] ^ k);   // position of the right neighbour in the other colour
-    s = s + P[right] * f[2];
-    s = s + P[right - 1] * f[3];
+    const int* nb = c.nb[k][j];
+    float s = P[nb[0]] * f[0] + P[nb[1]] * f[1];
+    s = s + P[nb[2]] * f[2];
+    s = s + P[nb[3]] * f[3];
     if constexpr (DIM == 3) {
-        s = s + P[q + g.ncol] * f[4];
-        s = s + P[q - g.ncol] * f[5];
+        s = s + P[nb[4]] * f[4];
+        s = s + P[nb[5]] * f[5];
     }
     return s;
 }
@@ -273,7 +300,7 @@ SS_D void split_sweeps(cg::cluster_group& cl, const Slab& g, const Cells<K>& c, 
         for (int k = 0; k < 2; ++k) {
             float v[K];
 #pragma unroll
-            for (int j = 0; j < K; ++j) v[j] = cell_sum<DIM>(g, c, k, j) - c.r[k][j] * g.hh;
+            for (int j = 0; j < K; ++j) v[j] = cell_sum<DIM>(c, k, j) - c.r[k][j] * g.hh;
 #pragma unroll
             for (int j = 0; j < K; ++j) {
                 float q = div_recip(v[j], c.fs[k][j], c.yr[k][j]);
@@ -299,7 +326,7 @@ SS_D bool solo_loop(const Slab& g, const Cells<K>& c, int iterations, int nt) {
         for (int k = 0; k < 2; ++k) {
             float v[K];
 #pragma unroll
-            for (int j = 0; j < K; ++j) v[j] = cell_sum<DIM>(g, c, k, j) - (c.act[k][j] ? c.r[k][j] * g.hh : -1.f);
+            for (int j = 0; j < K; ++j) v[j] = cell_sum<DIM>(c, k, j) - (c.act[k][j] ? c.r[k][j] * g.hh : -1.f);
 #pragma unroll
             for (int j = 0; j < K; ++j) {
                 const float q = EXACT ? div_exact(v[j], c.fs[k][j]) : div_recip(v[j], c.fs[k][j], c.yr[k][j]);
@@ -348,7 +375,7 @@ SS_D void slab_residual(const Slab& g, const Cells<K>& c, int fine, bool quirks,
         for (int k = 0; k < 2; ++k) {
             if (!c.in[k][j]) continue;
             const int q = threadIdx.x + j * kThreads;
-            const float lap = cell_sum<DIM>(g, c, k, j) - c.fr[k][j] * F[(k ? g.w[1] : g.w[0]) + q];
+            const float lap = cell_sum<DIM>(c, k, j) - c.fr[k][j] * F[(k ? g.w[1] : g.w[0]) + q];
             float res = c.r[k][j] - (g.inv_hh != 0.f ? lap * g.inv_hh : lap / g.hh);
             if (!c.live[k][j]) res = 0.f;
             if (quirks) {
@@ -589,7 +616,7 @@ SS_D void adj_sweeps_slab(cg::cluster_group* cl, const Slab& g, const Cells<K>& 
             float v[K];
 #pragma unroll
             for (int j = 0; j < K; ++j)
-                v[j] = it == 0 && k == 1 ? pb[k][j] : pb[k][j] + ws[k][j] * cell_sum<DIM>(g, c, k, j);
+                v[j] = it == 0 && k == 1 ? pb[k][j] : pb[k][j] + ws[k][j] * cell_sum<DIM>(c, k, j);
 #pragma unroll
             for (int j = 0; j < K; ++j) {
                 float t = div_recip(v[j], c.fs[k][j], c.yr[k][j]);
@@ -608,7 +635,7 @@ SS_D void adj_sweeps_slab(cg::cluster_group* cl, const Slab& g, const Cells<K>& 
     }
     if (iterations > 0)
 #pragma unroll
-        for (int j = 0; j < K; ++j) pb[1][j] += ws[1][j] * cell_sum<DIM>(g, c, 1, j);
+        for (int j = 0; j < K; ++j) pb[1][j] += ws[1][j] * cell_sum<DIM>(c, 1, j);
 }
 
 // One visit of level l: on the way down the post-smoothing's transpose (the
@@ -777,10 +804,10 @@ static int level_planes(const ss_sim* s, int l, int ctas, int* solo) {
     return (long long)planes * ncol <= kCells * kThreads ? planes : 0;
 }
 
-// shared memory in floats of levels L.. on `ctas` CTAs: pressures, prolongation
+// shared memory in floats of levels L.. on `ctas` CTAs: zeros, pressures, prolongation
 // taps, then the residuals / staged coarse planes / the matrix product's vector
 static long long coarse_floats(const ss_sim* s, int L, int ctas, long long* nw, long long* ntap) {
-    long long w = 0, taps = 0, fine = 0;
+    long long w = kZeros, taps = 0, fine = 0;
     for (int l = L; l < s->levels; ++l) {
         int solo;
         const int planes = level_planes(s, l, ctas, &solo);
@@ -904,7 +931,7 @@ static int coarse_args(const ss_sim* s, const ss_mg_schedule& mg, int L, T* cons
     b.nlev = s->levels - L;
     long long nw = 0, taps = 0;
     *floats = coarse_floats(s, L, ctas, &nw, &taps);
-    int w = 0, tap = 0;
+    int w = kZeros, tap = 0;
     for (int l = 0; l < b.nlev; ++l) {
         const ss::Level& lv = s->lv[L + l];
         for (int d = 0; d < 3; ++d) b.lv[l].n[d] = lv.n[d];
@@ -1055,8 +1082,9 @@ static int launch_response(ss_sim* s, int iters, float* D, int layout, const int
     if (n > kCoarseResponseMax || !b.lv[0].planes)
         return set_error(SS_E_INVALID, "coarsest level too large for its response matrix");
     b.lv[0].hh = lv.hh;
+    b.lv[0].w = kZeros;
     b.alpha[0] = s->alpha[l];
-    b.nw = s->dim == 3 ? slab_floats<3>(lv.n, b.lv[0].planes) : slab_floats<2>(lv.n, b.lv[0].planes);
+    b.nw = kZeros + (s->dim == 3 ? slab_floats<3>(lv.n, b.lv[0].planes) : slab_floats<2>(lv.n, b.lv[0].planes));
     b.n_coarse = iters;
     b.oob_smooth = b.oob_resid = smooth_oob(s, 0);
     const size_t smem = (size_t)b.nw * sizeof(float);
