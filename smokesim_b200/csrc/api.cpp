@@ -968,7 +968,11 @@ static int run_solve_chain(ss_sim* s, const ss_params* p, const StepConsts& c, i
 }
 
 static int chain_state(ss_sim* s, const ss_params* p, int depth, cudaStream_t st) {
-    if (!s->device_loop || !graphs_ok(s, st)) return -1;
+    // On the legacy default stream the host loop: it records one step a parity, on the
+    // second solve, where the chain records nine (two frames of a new simulation,
+    // 256^2 1.5 against 2.9 ms, 192x128x160 5.9 against 8.2; later ones 0.38 either way
+    // and 1.37 against 1.47).
+    if (!s->device_loop || !st || !graphs_ok(s, st)) return -1;
     // the chain is recorded by the first solve: a host loop of 46 launches and a
     // read-back a step costs it more (two frames of a new 128^3 rollout 8.8
     // against 10.3 ms)
