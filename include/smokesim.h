@@ -221,8 +221,10 @@ int ss_run_physics_step(ss_sim* sim, const ss_params* params, int nsteps, void* 
 /* Statistics of the last ss_run_physics_step call.  A step that neither
  * collects statistics nor solves to a tolerance returns SS_OK before its
  * kernels ran: a CUDA error of theirs is reported by the next call that waits
- * for the device (ss_get_field with a host destination, or the step itself when
- * it collects statistics or solves to a tolerance). */
+ * for the device - ss_get_field with a host destination, the step itself when
+ * it collects statistics or solves to a tolerance, and after an FP32 solve that
+ * none of these has waited for also ss_get_stats, which waits for the default
+ * stream (and with it for every stream that the default stream waits for). */
 int ss_get_stats(ss_sim* sim, ss_stats* out);
 
 /* ---- individual stages (reference common/physics/grid.h:37-68) -------------- */

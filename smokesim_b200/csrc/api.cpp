@@ -548,6 +548,7 @@ int ss_get_field(ss_sim* s, int f, float* host, size_t count, void* stream) {
     if (count != n) return set_error(SS_E_INVALID, "element count does not match the field");
     CU(cudaMemcpyAsync(host, d, n * sizeof(float), cudaMemcpyDeviceToHost, st), "get_field");
     CU(cudaStreamSynchronize(st), "get_field sync");
+    s->unchecked = 0;
     return SS_OK;
 }
 
@@ -661,6 +662,7 @@ static int v_cycle_rec(ss_sim* s, const StepConsts& c, const ss_mg_schedule& mg,
 static int read_slots(ss_sim* s, cudaStream_t st) {
     CU(cudaMemcpyAsync(s->red.host, s->red.out, SLOT_COUNT * sizeof(double), cudaMemcpyDeviceToHost, st), "slots");
     CU(cudaStreamSynchronize(st), "slots sync");
+    s->unchecked = 0;
     return SS_OK;
 }
 
@@ -1074,6 +1076,7 @@ static int pressure_solve(ss_sim* s, const ss_params* p, const StepConsts& c, cu
     s->solves += 1;
     if (mg.precision != SS_PREC_FP32) return pressure_solve_mixed(s, p, c, st, defer_p0);
     s->p64_valid = 0;
+    s->unchecked = 1;
     const bool tol_mode = mg.tol > 0.0;
     const bool stats = p->collect_stats || tol_mode;
     TRY(ensure_pyramid(s, st));
@@ -1271,7 +1274,8 @@ int ss_set_force_field(ss_sim* s, int n, const float* field, void* stream) {
 int ss_get_stats(ss_sim* s, ss_stats* out) {
     if (!s || !out) return set_error(SS_E_INVALID, "NULL argument");
     *out = s->st;
-    return SS_OK;
+    // a caller may have no other check of an FP32 step than this
+    return s->unchecked ? read_slots(s, nullptr) : SS_OK;
 }
 
 // ------------------------------------------------------------ single stages

@@ -141,6 +141,7 @@ struct ss_sim {
     int pyramid_dirty = 1;
 
     ss_stats st{};
+    int unchecked = 0;         // an FP32 solve ran since the host last waited for the device
     long long nlaunch = 0;     // kernels launched since the counter was reset
     // mixed solve: the coarsest level by its response matrix instead of its
     // n_coarse sweeps (levels of at most kCoarseResponseMax cells)
