@@ -900,8 +900,11 @@ static int largest_cluster() {
 // Largest cluster this device places (16 is not a portable size), else one
 // CTA; the first level that then runs in k_coarse.  Called outside any capture.
 int coarse_setup(ss_sim* s) {
-    // the attributes and the occupancy query take milliseconds together, and
-    // both are the device's: once per process and device
+    // the attributes are the context's: for every simulation
+    const cudaError_t e = s->dim == 3 ? coarse_attributes_all<3>() : coarse_attributes_all<2>();
+    if (e != cudaSuccess) return check_cuda(e, "coarse cluster attributes");
+    // the occupancy query takes milliseconds and its answer is the device's: once
+    // per process and device
     static std::mutex mu;
     static std::map<int, int> known;   // 4 * device + dim -> CTAs
     int dev = 0;
@@ -909,11 +912,7 @@ int coarse_setup(ss_sim* s) {
     {
         std::lock_guard<std::mutex> lock(mu);
         int& c = known[4 * dev + s->dim];
-        if (!c) {
-            const cudaError_t e = s->dim == 3 ? coarse_attributes_all<3>() : coarse_attributes_all<2>();
-            if (e != cudaSuccess) return check_cuda(e, "coarse cluster attributes");
-            c = s->dim == 3 ? largest_cluster<3>() : largest_cluster<2>();
-        }
+        if (!c) c = s->dim == 3 ? largest_cluster<3>() : largest_cluster<2>();
         s->coarse_max_ctas = s->use_cluster ? c : 1;
     }
     s->coarse_from = s->levels;
