@@ -364,7 +364,9 @@ typedef struct ss_render_desc {
 /* defaults of the reference's graphics_settings (common/graphics/graphics.c:9-25)
  * and a camera outside the +z face looking at the box centre */
 int ss_render_default(const ss_sim* sim, int width, int height, ss_render_desc* out);
-/* rgba: width*height*4 bytes, device memory when on_device, else host */
+/* rgba: width*height*4 bytes, device memory when on_device, else host.  In 3D a
+ * camera_target that equals camera_pos, or a direction parallel to camera_up, is
+ * SS_E_INVALID; a ray takes at most 2^24 samples */
 int ss_render(ss_sim* sim, const ss_render_desc* desc, uint8_t* rgba, int on_device, void* stream);
 
 /* ---- snapshots ---------------------------------------------------------- */

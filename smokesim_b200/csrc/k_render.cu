@@ -125,6 +125,8 @@ SS_D unsigned char to_unorm8(float v) {
     return (unsigned char)(v * 255.f + 0.5f);
 }
 
+constexpr int kMaxSteps = 1 << 24;   // samples a ray: a step below 2^-24 of t does not move it
+
 // i-th of n places from the middle outwards
 SS_D int centre_out(int i, int n) { return (n - 1) / 2 + ((i & 1) ? (i + 1) / 2 : -(i / 2)); }
 
@@ -163,7 +165,9 @@ __global__ void __launch_bounds__(128) k_raymarch(RenderArgs a, uchar4* __restri
         out[o] = make_uchar4(0, 0, 0, 0);
         return;
     }
-    const int steps = (int)((exit_ - enter) / a.step) + 1;
+    // bounded where the step is tiny against the chord: the march must end
+    const float count = (exit_ - enter) / a.step;
+    const int steps = count >= (float)kMaxSteps ? kMaxSteps : (int)count + 1;
     const float noise = fract_(sinf(u * 12.9898f + v * 78.233f) * 43758.5453f);
     float t = enter + noise * a.step;
     // phase_function(g, dot(-dir, light)) * 3, with the shader's PI = 3.14
@@ -300,6 +304,12 @@ int ss_render(ss_sim* s, const ss_render_desc* d, uint8_t* rgba, int on_device, 
     cross3(a.fwd, d->camera_up, a.right);
     normalize3(a.right);
     cross3(a.right, a.fwd, a.up);
+    // a direction that is 0, parallel to camera_up or too long to normalise: its rays
+    // would be NaN, which no box test stops
+    if (s->dim == 3)
+        for (int k = 0; k < 3; ++k)
+            if (!std::isfinite(a.fwd[k]) || !std::isfinite(a.right[k]) || !std::isfinite(a.up[k]))
+                return set_error(SS_E_INVALID, "camera direction is zero or parallel to camera_up");
     normalize3(a.light);
     a.tan_half = tanf(0.5f * d->fov_y);
     a.aspect = (float)d->width / (float)d->height;
