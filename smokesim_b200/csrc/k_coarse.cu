@@ -173,11 +173,13 @@ SS_D void load_cells(const Slab& g, const float* __restrict__ alpha, const T* r,
         e[4] = DIM == 3 && c.m[j] + 1 < g.nm;
         e[5] = DIM == 3 && c.m[j] > 0;
     };
-    // A neighbour outside the grid is read as 0, from the bank that its place in the
-    // packed order has: no test in the sweeps and no bank conflict.  In 3D
-    // formed after the loads are issued (reverse pass of a 64^3 solve of 8 V-cycles
-    // 1661 us, 1708 before them), in 2D before them (8 V-cycles at 256^2 with 16-bit
-    // storage 511 us; 559 after them, where those forms spill).
+    // A neighbour outside the grid is read as 0, from a bank that no other lane reads:
+    // no test in the sweeps and no bank conflict.  Past the end of a row that is the
+    // bank of the row's other end: that of its place in the packed order is the next
+    // row's, whose lane may be reading there (8^3: 7 cycles more of 207 a half-sweep).
+    // In 3D the places are formed after the loads are issued (reverse pass of a 64^3
+    // solve of 8 V-cycles 1661 us, 1708 before them), in 2D before them (8 V-cycles at
+    // 256^2 with 16-bit storage 511 us; 559 after them, where those forms spill).
     auto places = [&](int k, int j) {
         bool e[6];
         edges(k, j, e);
@@ -186,8 +188,8 @@ SS_D void load_cells(const Slab& g, const float* __restrict__ alpha, const T* r,
         int* nb = c.nb[k][j];
         nb[0] = place(ts, e[0]);
         nb[1] = place(-ts, e[1]);
-        nb[2] = place(right, e[2]);
-        nb[3] = place(right - 1, e[3]);
+        nb[2] = place(e[2] ? right : right - g.hx, e[2]);
+        nb[3] = place(e[3] ? right - 1 : right - 1 + g.hx, e[3]);
         if constexpr (DIM == 3) {
             nb[4] = place(g.ncol, e[4]);
             nb[5] = place(-g.ncol, e[5]);
