@@ -1,6 +1,8 @@
-// coarse_level.cuh - per-cell multigrid operators of the coarse levels, shared
-// by the per-level kernels (k_mg.cu) and the one-launch lower V-cycle
-// (k_coarse.cu), so that a level gives the same values wherever it runs.
+// coarse_level.cuh - per-cell multigrid operators of the per-level kernels
+// (k_mg.cu), the out-of-grid rules and the coarsest level's matrix product, which
+// the one-launch lower V-cycle (k_coarse.cu) uses too.  That one sums its cells from
+// shared memory by code of its own, in the order of smooth_cell and residual_cell;
+// the tests hold the two to the same bits.
 #pragma once
 
 #include "common.cuh"
@@ -35,21 +37,10 @@ static inline float smooth_oob(const ss_sim* s, int quirks) { return quirks ? 0.
 static inline float resid_oob(const ss_sim* s, int quirks) { return quirks ? 1.f : (s->enclosed ? 1.f : 0.f); }
 
 // ------------------------------------------------------------------ smoother
-// A level value as float; CG reads through L2 only (ld.global.cg), for
-// arrays that other blocks of the same launch may have written since this SM
-// last cached them (L1 is not coherent across SMs).
-template <bool CG, typename T>
-SS_D float ldv(const T* p) {
-    if constexpr (CG) return ld(__ldcg(p));
-    else return ld(*p);
-}
-
 // smooth.comp:79-136 (2D :74-123): red-black Gauss-Seidel in place; solid
 // cells and cells without fluid neighbours are skipped; out of grid = fluid
 // with p = 0.
-// R: the type whose rounding every stored pressure gets (== T for global
-// arrays).
-template <int DIM, bool L0, typename T = float, typename R = T, bool CG = false>
+template <int DIM, bool L0, typename T = float>
 SS_D void smooth_cell(const MGArgsT<T>& a, int x, int y, int z) {
     const int nx = a.nx, ny = a.ny, nz = a.nz;
     const int c = idx3(x, y, z, nx, ny);
@@ -58,13 +49,13 @@ SS_D void smooth_cell(const MGArgsT<T>& a, int x, int y, int z) {
     float p_top, p_bottom, p_right, p_left, p_front = 0.f, p_back = 0.f;
     auto load_p = [&]() {
         const T* P = a.p;
-        p_top = y + 1 < ny ? ldv<CG>(P + c + nx) : 0.f;
-        p_bottom = y > 0 ? ldv<CG>(P + c - nx) : 0.f;
-        p_right = x + 1 < nx ? ldv<CG>(P + c + 1) : 0.f;
-        p_left = x > 0 ? ldv<CG>(P + c - 1) : 0.f;
+        p_top = y + 1 < ny ? ld(P[c + nx]) : 0.f;
+        p_bottom = y > 0 ? ld(P[c - nx]) : 0.f;
+        p_right = x + 1 < nx ? ld(P[c + 1]) : 0.f;
+        p_left = x > 0 ? ld(P[c - 1]) : 0.f;
         if constexpr (DIM == 3) {
-            p_front = z + 1 < nz ? ldv<CG>(P + c + nx * ny) : 0.f;
-            p_back = z > 0 ? ldv<CG>(P + c - nx * ny) : 0.f;
+            p_front = z + 1 < nz ? ld(P[c + nx * ny]) : 0.f;
+            p_back = z > 0 ? ld(P[c - nx * ny]) : 0.f;
         }
     };
     if constexpr (L0) {
@@ -92,9 +83,7 @@ SS_D void smooth_cell(const MGArgsT<T>& a, int x, int y, int z) {
             a_f = z + 1 < nz ? a.alpha[c + nx * ny] : a.oobA;
             a_k = z > 0 ? a.alpha[c - nx * ny] : a.oobA;
         }
-        r_c = ldv<CG>(a.r + c);
-        // the neighbours' pressures too: with CG they come from L2, and
-        // issuing them here keeps the cell to one memory round trip
+        r_c = ld(a.r[c]);
         load_p();
         if (a_c >= 1.f) return;
         f_top = 1.f - a_t;
@@ -120,13 +109,13 @@ SS_D void smooth_cell(const MGArgsT<T>& a, int x, int y, int z) {
     float pn;
     if constexpr (L0) pn = (p_sum - a.rho_h * a.div0[c] / a.dt) / f_sum;
     else pn = (p_sum - r_c * a.hh) / f_sum;
-    a.p[c] = st<T>(rnd<R>(pn));
+    a.p[c] = st<T>(pn);
 }
 
 // ------------------------------------------------------------------ residual
 // compute_residual.comp:77-130 (2D :72-117): r = b - (sum_f p_nb - f_sum p)/h^2,
 // out of grid = solid; level 0 takes b = rho*div/(dt*h).
-template <int DIM, bool L0, typename T = float, bool CG = false>
+template <int DIM, bool L0, typename T = float>
 SS_D float residual_cell(const MGArgsT<T>& a, int x, int y, int z) {
     const int nx = a.nx, ny = a.ny, nz = a.nz;
     const int c = idx3(x, y, z, nx, ny);
@@ -134,15 +123,15 @@ SS_D float residual_cell(const MGArgsT<T>& a, int x, int y, int z) {
     float p_top, p_bottom, p_right, p_left, p_front = 0.f, p_back = 0.f, p_c, old;
     const T* P = a.p;
     auto load_p = [&]() {
-        p_top = y + 1 < ny ? ldv<CG>(P + c + nx) : 0.f;
-        p_bottom = y > 0 ? ldv<CG>(P + c - nx) : 0.f;
-        p_right = x + 1 < nx ? ldv<CG>(P + c + 1) : 0.f;
-        p_left = x > 0 ? ldv<CG>(P + c - 1) : 0.f;
+        p_top = y + 1 < ny ? ld(P[c + nx]) : 0.f;
+        p_bottom = y > 0 ? ld(P[c - nx]) : 0.f;
+        p_right = x + 1 < nx ? ld(P[c + 1]) : 0.f;
+        p_left = x > 0 ? ld(P[c - 1]) : 0.f;
         if constexpr (DIM == 3) {
-            p_front = z + 1 < nz ? ldv<CG>(P + c + nx * ny) : 0.f;
-            p_back = z > 0 ? ldv<CG>(P + c - nx * ny) : 0.f;
+            p_front = z + 1 < nz ? ld(P[c + nx * ny]) : 0.f;
+            p_back = z > 0 ? ld(P[c - nx * ny]) : 0.f;
         }
-        p_c = ldv<CG>(P + c);
+        p_c = ld(P[c]);
     };
     if constexpr (L0) {
         const uint8_t fl = a.flags[c];
@@ -172,7 +161,7 @@ SS_D float residual_cell(const MGArgsT<T>& a, int x, int y, int z) {
             a_k = z > 0 ? a.alpha[c - nx * ny] : a.oobA;
         }
         load_p();
-        old = ldv<CG>(a.r + c);
+        old = ld(a.r[c]);
         if (a_c >= 1.f) return 0.f;
         f_top = 1.f - a_t;
         f_bottom = 1.f - a_b;
@@ -195,17 +184,14 @@ SS_D float residual_cell(const MGArgsT<T>& a, int x, int y, int z) {
     return old - (p_sum - f_sum * p_c) / a.hh;
 }
 
-// T: storage type of the global level arrays; R: rounding of every value the
-// solve stores (T, or float for the FP32 solve).
 // Part of p_j = sum_i E[i n + j] r_i over i in [i0, i1), where E[i n + j] =
 // dp_j / dr_i of the coarsest level's n_coarse sweeps from p = 0
 // (k_coarse_response, layout 1): eight partial sums taken round-robin
 // ((i - i0) mod 8), added pairwise, so the oracle can repeat the order.  Two
 // rounds of eight independent loads are in flight per step (the matrix
 // streams from L2).
-// r: the level's right-hand side, in shared memory or (CG) global.
-template <bool CG = false, typename RT>
-SS_D float coarse_product(const float* __restrict__ E, const RT* r, int n, int j, int i0, int i1) {
+// r: the level's right-hand side, in shared memory.
+SS_D float coarse_product(const float* __restrict__ E, const float* r, int n, int j, int i0, int i1) {
     float a[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     const float* e = E + j;
     int i = i0;
@@ -214,11 +200,11 @@ SS_D float coarse_product(const float* __restrict__ E, const RT* r, int n, int j
 #pragma unroll
         for (int k = 0; k < 16; ++k) v[k] = __ldg(e + (size_t)(i + k) * n);
 #pragma unroll
-        for (int k = 0; k < 16; ++k) a[k & 7] += v[k] * ldv<CG>(r + i + k);
+        for (int k = 0; k < 16; ++k) a[k & 7] += v[k] * r[i + k];
     }
 #pragma unroll
     for (int k = 0; k < 16; ++k)
-        if (i + k < i1) a[k & 7] += __ldg(e + (size_t)(i + k) * n) * ldv<CG>(r + i + k);
+        if (i + k < i1) a[k & 7] += __ldg(e + (size_t)(i + k) * n) * r[i + k];
     return ((a[0] + a[1]) + (a[2] + a[3])) + ((a[4] + a[5]) + (a[6] + a[7]));
 }
 
@@ -238,23 +224,22 @@ SS_D int coarse_parts(int n) {
 // coalesced); its sum goes to part[q n + j].  Phase 2: value j folds its
 // slices as a tree, v[q] += v[q + o] for o = parts/2 .. 1, rounds the result
 // as R and stores it as PT.  `part` holds parts * n <= kProductLanes floats.
-template <bool CG, typename RT>
-SS_D void coarse_matrix_partials(const float* __restrict__ E, const RT* r, float* part, int n, int tid,
+SS_D void coarse_matrix_partials(const float* __restrict__ E, const float* r, float* part, int n, int tid,
                                  int nthreads) {
     const int parts = coarse_parts(n), chunk = (n + parts - 1) / parts;
     for (int t = tid; t < parts * n; t += nthreads) {
         const int q = t / n, j = t % n;
-        part[t] = coarse_product<CG>(E, r, n, j, q * chunk, min(n, (q + 1) * chunk));
+        part[t] = coarse_product(E, r, n, j, q * chunk, min(n, (q + 1) * chunk));
     }
 }
 
-template <bool CG, typename R, typename PT>
+template <typename R, typename PT>
 SS_D void coarse_matrix_fold(const float* part, PT* p, int n, int tid, int nthreads) {
     const int parts = coarse_parts(n);
     for (int j = tid; j < n; j += nthreads) {
         float v[32];
 #pragma unroll
-        for (int q = 0; q < 32; ++q) v[q] = q < parts ? ldv<CG>(part + q * n + j) : 0.f;
+        for (int q = 0; q < 32; ++q) v[q] = q < parts ? __ldcg(part + q * n + j) : 0.f;
 #pragma unroll
         for (int o = 16; o >= 1; o >>= 1)
             if (o < parts) {

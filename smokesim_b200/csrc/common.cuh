@@ -56,35 +56,8 @@ SS_D float fetch_b(const float* __restrict__ a, int ax, int ay, int az, int x, i
     return __ldg(a + idx3(x, y, z, ax, ay));
 }
 
-// GL_LINEAR + CLAMP_TO_BORDER at texel-space coordinate (texel centres at integers).
-template <int DIM>
-SS_D float sample_border(const float* __restrict__ a, int ax, int ay, int az, float tx, float ty, float tz,
-                         float border) {
-    tx = clampt(tx, -2.f, (float)(ax + 1));
-    ty = clampt(ty, -2.f, (float)(ay + 1));
-    float fx = floorf(tx), fy = floorf(ty);
-    int x0 = (int)fx, y0 = (int)fy;
-    float wx = tx - fx, wy = ty - fy;
-    if constexpr (DIM == 2) {
-        float c00 = fetch_b(a, ax, ay, 1, x0, y0, 0, border), c10 = fetch_b(a, ax, ay, 1, x0 + 1, y0, 0, border);
-        float c01 = fetch_b(a, ax, ay, 1, x0, y0 + 1, 0, border), c11 = fetch_b(a, ax, ay, 1, x0 + 1, y0 + 1, 0, border);
-        return lerp_(lerp_(c00, c10, wx), lerp_(c01, c11, wx), wy);
-    } else {
-        tz = clampt(tz, -2.f, (float)(az + 1));
-        float fz = floorf(tz);
-        int z0 = (int)fz;
-        float wz = tz - fz;
-        float c000 = fetch_b(a, ax, ay, az, x0, y0, z0, border), c100 = fetch_b(a, ax, ay, az, x0 + 1, y0, z0, border);
-        float c010 = fetch_b(a, ax, ay, az, x0, y0 + 1, z0, border), c110 = fetch_b(a, ax, ay, az, x0 + 1, y0 + 1, z0, border);
-        float c001 = fetch_b(a, ax, ay, az, x0, y0, z0 + 1, border), c101 = fetch_b(a, ax, ay, az, x0 + 1, y0, z0 + 1, border);
-        float c011 = fetch_b(a, ax, ay, az, x0, y0 + 1, z0 + 1, border), c111 = fetch_b(a, ax, ay, az, x0 + 1, y0 + 1, z0 + 1, border);
-        float c0 = lerp_(lerp_(c000, c100, wx), lerp_(c010, c110, wx), wy);
-        float c1 = lerp_(lerp_(c001, c101, wx), lerp_(c011, c111, wx), wy);
-        return lerp_(c0, c1, wz);
-    }
-}
-
-// Tap positions and weights of one border sample, shared by several channels.
+// Tap positions and weights of one sample with GL_LINEAR and CLAMP_TO_BORDER at a
+// texel-space coordinate (texel centres at integers), shared by several channels.
 struct Taps {
     int x0, y0, z0;
     float wx, wy, wz;
@@ -127,25 +100,9 @@ SS_D float sample_taps(const float* __restrict__ a, int ax, int ay, int az, cons
     }
 }
 
-// Velocity at grid-space point g (reference get_interpolated_velocity,
-// shaders3d/compute/advect_vx.comp:33-46).
-template <int DIM>
-SS_D void interp_velocity(const float* __restrict__ u, const float* __restrict__ v, const float* __restrict__ w,
-                          int nx, int ny, int nz, float gx, float gy, float gz, float out[3]) {
-    if constexpr (DIM == 2) {
-        out[0] = sample_border<2>(u, nx + 1, ny, 1, gx, gy - 0.5f, 0.f, 0.f);
-        out[1] = sample_border<2>(v, nx, ny + 1, 1, gx - 0.5f, gy, 0.f, 0.f);
-        out[2] = 0.f;
-    } else {
-        out[0] = sample_border<3>(u, nx + 1, ny, nz, gx, gy - 0.5f, gz - 0.5f, 0.f);
-        out[1] = sample_border<3>(v, nx, ny + 1, nz, gx - 0.5f, gy, gz - 0.5f, 0.f);
-        out[2] = sample_border<3>(w, nx, ny, nz + 1, gx - 0.5f, gy - 0.5f, gz, 0.f);
-    }
-}
-
-
 // ---------------------------------------------------------------------------
-// Specialised forms of sample_border at the points the kernels actually use.
+// Velocity (reference get_interpolated_velocity, shaders3d/compute/advect_vx.comp:33-46)
+// at the points the kernels use.
 // At a MAC face or cell centre every texel-space coordinate is an integer or
 // an integer + 1/2, so each linear weight is exactly 0 or 0.5.  A weight-0
 // lerp a*(1-0) + b*0 equals a (for finite b), so skipping those taps gives the
@@ -339,7 +296,7 @@ SS_D float div_by_count(float a, int f) {
 // Fluid mask byte of a level-0 cell: bit 0 the cell is fluid, bits 1-6 the
 // +y,-y,+x,-x,+z,-z neighbour is fluid (out of grid: fluid on an open grid,
 // solid on an enclosed one).  Zero - a load outside the grid - reads as
-// "not fluid", so tile kernels need no bounds checks.
+// "not fluid".
 enum : uint8_t {
     M_FLUID = 1u << 0,
     M_TOP = 1u << 1,

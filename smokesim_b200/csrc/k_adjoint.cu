@@ -1314,38 +1314,6 @@ int adj_v_cycle(ss_sim* s, const StepConsts& c, const ss_mg_schedule& mg, const 
     return adj_v_cycle_rec(s, c, mg, 0, w, st);
 }
 
-// level-0 operator L p = sum_j w_j p_j - d p (fluid cells), for the mixed
-// solve's refinement transpose: pbar -= k * L(rbar) (L is symmetric)
-template <int DIM>
-__global__ void __launch_bounds__(256) k_adj_apply_laplacian(const float* __restrict__ rb, const uint8_t* __restrict__ fmask,
-                                                             int nx, int ny, int nz, float k, float* __restrict__ pbar) {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
-    const int y = blockIdx.y * blockDim.y + threadIdx.y;
-    const int z = blockIdx.z * blockDim.z + threadIdx.z;
-    if (x >= nx || y >= ny || z >= nz) return;
-    const int c = idx3(x, y, z, nx, ny);
-    const uint8_t m = fmask[c];
-    if (!(m & M_FLUID)) return;
-    float s = 0.f;
-    if ((m & M_TOP) && y + 1 < ny) s += rb[c + nx];
-    if ((m & M_BOTTOM) && y > 0) s += rb[c - nx];
-    if ((m & M_RIGHT) && x + 1 < nx) s += rb[c + 1];
-    if ((m & M_LEFT) && x > 0) s += rb[c - 1];
-    if constexpr (DIM == 3) {
-        if ((m & M_FRONT) && z + 1 < nz) s += rb[c + nx * ny];
-        if ((m & M_BACK) && z > 0) s += rb[c - nx * ny];
-    }
-    pbar[c] -= k * (s - (float)__popc(m & 0x7Eu) * rb[c]);
-}
-
-int adj_apply_laplacian(ss_sim* s, const float* rb, float k, float* pbar, cudaStream_t st) {
-    dim3 g = grid_of(s->nx, s->ny, s->nz, kB);
-    if (s->dim == 3) k_adj_apply_laplacian<3><<<g, kB, 0, st>>>(rb, s->fmask, s->nx, s->ny, s->nz, k, pbar);
-    else k_adj_apply_laplacian<2><<<g, kB, 0, st>>>(rb, s->fmask, s->nx, s->ny, s->nz, k, pbar);
-    s->nlaunch += 1;
-    return check_cuda(cudaGetLastError(), "k_adj_apply_laplacian");
-}
-
 int adj_vorticity(ss_sim* s, const StepConsts& c, const float* vort, float* const vb[3], float* wdir, float* dbar,
                   float* wbar, cudaStream_t st) {
     dim3 g = grid_of(s->nx, s->ny, s->nz, kB);

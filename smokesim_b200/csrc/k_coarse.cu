@@ -581,11 +581,11 @@ __global__ void __launch_bounds__(kThreads) k_coarse(const __grid_constant__ Coa
     if (b.cmat) {
         const int n = b.lv[last].n[0] * b.lv[last].n[1] * b.lv[last].n[2];
         cl.sync();
-        for (int i = threadIdx.x; i < n; i += kThreads) F[b.fine + i] = ldv<true>(b.r[last] + i);
+        for (int i = threadIdx.x; i < n; i += kThreads) F[b.fine + i] = ld(__ldcg(b.r[last] + i));
         __syncthreads();
-        coarse_matrix_partials<false>(b.cmat, F + b.fine, b.cpart, n, rank * kThreads + (int)threadIdx.x, ctas * kThreads);
+        coarse_matrix_partials(b.cmat, F + b.fine, b.cpart, n, rank * kThreads + (int)threadIdx.x, ctas * kThreads);
         cl.sync();
-        coarse_matrix_fold<true, R>(b.cpart, b.p[last], n, rank * kThreads + (int)threadIdx.x, ctas * kThreads);
+        coarse_matrix_fold<R>(b.cpart, b.p[last], n, rank * kThreads + (int)threadIdx.x, ctas * kThreads);
         cl.sync();
     } else {
         run(last, false);
@@ -778,9 +778,9 @@ __global__ void __launch_bounds__(kThreads) k_adj_coarse(const __grid_constant__
         const int n = b.lv[last].n[0] * b.lv[last].n[1] * b.lv[last].n[2];
         for (int i = threadIdx.x; i < n; i += kThreads) F[b.fine + i] = __ldcg(b.p[last] + i);
         __syncthreads();
-        coarse_matrix_partials<false>(b.cmat, F + b.fine, b.cpart, n, first, threads);
+        coarse_matrix_partials(b.cmat, F + b.fine, b.cpart, n, first, threads);
         cl.sync();
-        coarse_matrix_fold<true, float>(b.cpart, b.r[last], n, first, threads);
+        coarse_matrix_fold<float>(b.cpart, b.r[last], n, first, threads);
         cl.sync();
     } else {
         run(last, false);

@@ -50,10 +50,6 @@ static FluidArgs fluid_args(ss_sim* s, const StepConsts& c) {
     return a;
 }
 
-SS_D bool solid_oob1(const uint8_t* __restrict__ f, int x, int y, int z, int nx, int ny, int nz) {
-    if (x < 0 || y < 0 || z < 0 || x >= nx || y >= ny || z >= nz) return true;
-    return f[idx3(x, y, z, nx, ny)] & F_SOLID;
-}
 SS_D bool solid_oob0(const uint8_t* __restrict__ f, int x, int y, int z, int nx, int ny, int nz) {
     if (x < 0 || y < 0 || z < 0 || x >= nx || y >= ny || z >= nz) return false;
     return f[idx3(x, y, z, nx, ny)] & F_SOLID;

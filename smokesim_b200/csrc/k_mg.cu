@@ -15,13 +15,6 @@
 
 namespace ss {
 
-#define TRY_CUDA_MG(x, what)                              \
-    do {                                                  \
-        const int _rc = check_cuda((x), what);            \
-        if (_rc != SS_OK) return _rc;                     \
-    } while (0)
-
-
 static MGArgs mg_args(ss_sim* s, const StepConsts& c, int L, float oobA) {
     MGArgs a;
     a.oobA = oobA;
@@ -76,7 +69,7 @@ int launch_smooth(ss_sim* s, const StepConsts& c, int L, int iterations, int qui
 // when WRITE_FINE, the reference's in-place residual), then restrict_residual
 // (restrict_residual.comp:40-64, 2D :40-59) into the next level when
 // WRITE_COARSE.  The grid also covers the fine cells left over by odd sizes.
-template <int DIM, bool L0, bool WRITE_FINE, bool WRITE_COARSE, typename T = float, bool CG = false>
+template <int DIM, bool L0, bool WRITE_FINE, bool WRITE_COARSE, typename T = float>
 SS_D void residual_restrict_cell(const MGArgsT<T>& a, T* __restrict__ rc, int cx, int cy, int cz, int X, int Y, int Z,
                                  T* __restrict__ pz = nullptr) {
     const int nx = a.nx, ny = a.ny, nz = a.nz;
@@ -92,7 +85,7 @@ SS_D void residual_restrict_cell(const MGArgsT<T>& a, T* __restrict__ rc, int cx
                 const int x = x0 + dx, y = y0 + dy, z = z0 + dz;
                 float res = 0.f;
                 if (x < nx && y < ny && z < nz) {
-                    res = residual_cell<DIM, L0, T, CG>(a, x, y, z);
+                    res = residual_cell<DIM, L0, T>(a, x, y, z);
                     if constexpr (WRITE_FINE) {
                         a.r[idx3(x, y, z, nx, ny)] = st<T>(res);
                         res = rnd<T>(res);
@@ -195,7 +188,7 @@ int launch_restrict(ss_sim* s, int L, cudaStream_t st) {
 // --------------------------------------------------------------- prolongation
 // prolong_pressure.comp:39-51: p_L += GL_LINEAR, CLAMP_TO_EDGE sample of
 // p_{L+1} at the fine cell centre, on every cell.
-template <int DIM, typename T = float, bool CG = false>
+template <int DIM, typename T = float>
 SS_D void prolong_cell(T* __restrict__ p, int ax, int ay, int az, const T* __restrict__ pc, int cx, int cy, int cz,
                        int x, int y, int z) {
     if (x >= ax || y >= ay || z >= az) return;
@@ -208,22 +201,22 @@ SS_D void prolong_cell(T* __restrict__ p, int ax, int ay, int az, const T* __res
     const int ya = min(max(y0, 0), cy - 1), yb = min(max(y0 + 1, 0), cy - 1);
     float s;
     if constexpr (DIM == 2) {
-        s = lerp_(lerp_(ldv<CG>(&pc[idx3(xa, ya, 0, cx, cy)]), ldv<CG>(&pc[idx3(xb, ya, 0, cx, cy)]), wx),
-                  lerp_(ldv<CG>(&pc[idx3(xa, yb, 0, cx, cy)]), ldv<CG>(&pc[idx3(xb, yb, 0, cx, cy)]), wx), wy);
+        s = lerp_(lerp_(ld(pc[idx3(xa, ya, 0, cx, cy)]), ld(pc[idx3(xb, ya, 0, cx, cy)]), wx),
+                  lerp_(ld(pc[idx3(xa, yb, 0, cx, cy)]), ld(pc[idx3(xb, yb, 0, cx, cy)]), wx), wy);
     } else {
         const float tz = (((float)z + 0.5f) / (float)az) * (float)cz - 0.5f;
         const float fz = floorf(tz);
         const int z0 = (int)fz;
         const float wz = tz - fz;
         const int za = min(max(z0, 0), cz - 1), zb = min(max(z0 + 1, 0), cz - 1);
-        const float c0 = lerp_(lerp_(ldv<CG>(&pc[idx3(xa, ya, za, cx, cy)]), ldv<CG>(&pc[idx3(xb, ya, za, cx, cy)]), wx),
-                               lerp_(ldv<CG>(&pc[idx3(xa, yb, za, cx, cy)]), ldv<CG>(&pc[idx3(xb, yb, za, cx, cy)]), wx), wy);
-        const float c1 = lerp_(lerp_(ldv<CG>(&pc[idx3(xa, ya, zb, cx, cy)]), ldv<CG>(&pc[idx3(xb, ya, zb, cx, cy)]), wx),
-                               lerp_(ldv<CG>(&pc[idx3(xa, yb, zb, cx, cy)]), ldv<CG>(&pc[idx3(xb, yb, zb, cx, cy)]), wx), wy);
+        const float c0 = lerp_(lerp_(ld(pc[idx3(xa, ya, za, cx, cy)]), ld(pc[idx3(xb, ya, za, cx, cy)]), wx),
+                               lerp_(ld(pc[idx3(xa, yb, za, cx, cy)]), ld(pc[idx3(xb, yb, za, cx, cy)]), wx), wy);
+        const float c1 = lerp_(lerp_(ld(pc[idx3(xa, ya, zb, cx, cy)]), ld(pc[idx3(xb, ya, zb, cx, cy)]), wx),
+                               lerp_(ld(pc[idx3(xa, yb, zb, cx, cy)]), ld(pc[idx3(xb, yb, zb, cx, cy)]), wx), wy);
         s = lerp_(c0, c1, wz);
     }
     const int i = idx3(x, y, z, ax, ay);
-    p[i] = st<T>(ldv<CG>(p + i) + s);
+    p[i] = st<T>(ld(p[i]) + s);
 }
 
 template <int DIM, typename T = float>

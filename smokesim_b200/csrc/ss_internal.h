@@ -1,6 +1,5 @@
 // ss_internal.h - device state of one grid and the kernel launchers.
 #pragma once
-#include <cuda.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -317,7 +316,6 @@ int adj_advect_smoke(ss_sim* s, const StepConsts& c, const float* const vel[3], 
 int adj_update(ss_sim* s, const StepConsts& c, float* const vb[3], float* pbar, cudaStream_t st);
 int adj_divergence(ss_sim* s, const float* dbar, float* const vb[3], cudaStream_t st);
 int adj_v_cycle(ss_sim* s, const StepConsts& c, const ss_mg_schedule& mg, const AdjScratch& w, cudaStream_t st);
-int adj_apply_laplacian(ss_sim* s, const float* rb, float k, float* pbar, cudaStream_t st);
 int adj_vorticity(ss_sim* s, const StepConsts& c, const float* vort, float* const vb[3], float* wdir, float* dbar,
                   float* wbar, cudaStream_t st);
 int adj_advect_velocity(ss_sim* s, const StepConsts& c, bool buoy, const float* const vel[3], const float* dens,
