@@ -30,10 +30,10 @@
 //    memory (L2).
 //
 // Measured on B200 (one V-cycle, schedule 2 + 2 sweeps, 80 coarsest, whole
-// launch): FP32 32^3, 16^3, 8^3 52 us (before: 16^3 and 8^3 in one block from
+// launch): FP32 32^3, 16^3, 8^3 51 us (before: 16^3 and 8^3 in one block from
 // shared memory 73 us, and 32^3 as tiled launches 63 us); FP16 storage with the
-// response matrix at 128^3 37 us (through global memory 54 us); a coarsest level
-// of 24x18x15 cells 86 us (in one block 875 us: 0.5 against 5.4 us a half-sweep).
+// response matrix at 128^3 43 us (through global memory 54 us); a coarsest level
+// of 24x18x15 cells 85 us (in one block 875 us: 0.5 against 5.4 us a half-sweep).
 //
 // The arithmetic per cell is that of smooth_cell / residual_cell (a neighbour
 // outside the grid is a 0 read from shared memory; its weight still counts in the

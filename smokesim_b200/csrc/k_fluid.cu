@@ -266,8 +266,8 @@ SS_D float mean4(float a, float b, float c, float d) {
 // are loaded once, before any test.  Bound by its instruction stream and the
 // latency of the gathers, which hit L1 (DRAM traffic is the 33 B a cell): six
 // blocks an SM, at the price of a few spilled words on the branch of the border
-// samples.  318 us at 256^3 (357 with clamped taps, a floor conversion and loads
-// per face; 402 at the four blocks that 62 registers allow), 73 at 160x192x144 (89).
+// samples.  325 us at 256^3 (357 with clamped taps, a floor conversion and loads
+// per face; 402 at the four blocks that 62 registers allow), 75 at 160x192x144 (89).
 template <int DIM, bool BUOY>
 __global__ void __launch_bounds__(256, 6) k_advect_velocity(FluidArgs a, TapLimits lim) {
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
@@ -778,9 +778,9 @@ constexpr int kUpdPlanes = 8;
 // One thread per cell column takes the cells' low faces, and the faces past the
 // last cell of a row or column beside them: a grid of nx x ny threads, where one of
 // (nx + 1) x (ny + 1) leaves a ninth of the warps of a 256-cell row nearly empty.
-// Bound by memory latency, six blocks an SM: 124 us at 256^3 with the FP64 pressure
+// Bound by memory latency, six blocks an SM: 122 us at 256^3 with the FP64 pressure
 // (178 with a face position a thread, a bounds test and a neighbour's flags per
-// face; 127 at five blocks), 17.4 at 128^3 in FP32 (25.5), 4.1 at 64^3 (5.4).
+// face; 127 at five blocks), 16.8 at 128^3 in FP32 (25.5), 4.1 at 64^3 (5.4).
 template <int DIM, typename P = float>
 __global__ void __launch_bounds__(256, 6) k_update_velocity(FluidArgs a, const P* __restrict__ p, int planes,
                                                          double k64 = 0.0, float* __restrict__ p0_out = nullptr) {

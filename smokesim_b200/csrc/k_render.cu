@@ -73,8 +73,8 @@ SS_D void smoke_edge(const RenderArgs& a, const float t[3], float rgb[3]) {
 }
 
 // Density between a point of the ray and the light.  Two samples at a time, their
-// loads in flight together (three: 260 us, six: 30 more); the march ends early once it has left
-// the box for good (every further sample is zero).
+// loads in flight together (235 us a picture; one at a time 237, three 250, six 272);
+// the march ends early once it has left the box for good (every further sample is zero).
 constexpr int kShadowBatch = 2;
 template <int NCH>
 SS_D float shadow(const RenderArgs& a, const float pos[3]) {
@@ -133,10 +133,9 @@ SS_D int centre_out(int i, int n) { return (n - 1) / 2 + ((i & 1) ? (i + 1) / 2 
 // A warp takes 8 x 4 pixels, whose rays stay together, and a block four warps, so
 // that a long ray holds few others' place; blocks go from the middle of the
 // picture, where the smoke is, outwards, so that the last ones end soon.  Bound by
-// its instructions: 234 us for 1024 x 1024 rays through 192^3 cells of dense smoke;
-// 464 with rows of 32 pixels in blocks of 256, one shadow sample at a time, IEEE
-// divisions and clamped taps (248e6 warp instructions against 177e6; 272 with rows
-// from the top).
+// its instructions (178e6 of warps, 79% of the issue slots): 235 us for 1024 x 1024 rays
+// through 192^3 cells of dense smoke; 464 with rows of 32 pixels in blocks of 256, one
+// shadow sample at a time, IEEE divisions and clamped taps; 272 with rows from the top.
 template <int NCH>
 __global__ void __launch_bounds__(128) k_raymarch(RenderArgs a, uchar4* __restrict__ out) {
     const int px = centre_out(blockIdx.x, gridDim.x) * 8 + (threadIdx.x & 7);
