@@ -35,6 +35,6 @@ def test_first_frames_on_the_default_stream(monkeypatch):
         return t
 
     two_frames("1"), two_frames("0")
-    # the quickest of nine, in turn: the box's other work only ever adds time
+    # the quickest of nine, in turn: the machine's other work only ever adds time
     t = np.array([[two_frames("1"), two_frames("0")] for _ in range(9)]).min(0)
     assert t[0] <= 1.4 * t[1], t
