@@ -20,7 +20,7 @@ def test_stats_wait_for_an_unchecked_fp32_solve(checked):
     done = torch.cuda.Event()
 
     def busy():
-        torch.cuda._sleep(100_000_000)     # some 50 ms on the default stream
+        torch.cuda._sleep(1_000_000_000)     # some 0.5 s on the default stream
         done.record()
         assert not done.query()
 
